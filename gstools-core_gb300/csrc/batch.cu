@@ -19,8 +19,7 @@
 //  * the whole sequence is allocation-free and host-synchronisation-free,
 //    so it is captured once into a CUDA graph and replayed.
 //
-// The autotuner picks the points per thread R, the modes per staged tile
-// (FP64 form) and the work-unit granularity (how finely modes are split) by
+// The autotuner picks the points per thread R and the work-unit granularity (how finely modes are split) by
 // timing each candidate on an evenly spaced sample of the cost-sorted queue
 // of this very ensemble, and caches the winner per ensemble shape.
 #include <cuda_runtime.h>
@@ -45,7 +44,7 @@ namespace {
 
 struct Cfg {
     int R = 4;          // points per thread
-    int tile = 8;       // modes per staged tile (FP64 form)
+    int tile = 8;       // modes per staged tile as the caller names it (FP64 form: always 32)
     int upb = 8;        // target work units per resident block
 };
 
@@ -100,7 +99,6 @@ struct gsc_batch {
     BatchUnit *d_units = nullptr;
     size_t units_cap = 0;
     int *d_counter = nullptr;
-    void *d_tab = nullptr;                   // FP64 form: W tables (double2)
     double *d_rec = nullptr;                 // FP64 form: mode records
     float *d_frec = nullptr;                 // mixed forms: records
     double *d_rec64 = nullptr;
@@ -131,7 +129,7 @@ struct gsc_batch {
         if (graph) cudaGraphDestroy(graph);
         if (cap_stream) cudaStreamDestroy(cap_stream);
         for (void *p : {static_cast<void *>(d_items), static_cast<void *>(d_prefix),
-                        static_cast<void *>(d_units), static_cast<void *>(d_counter), d_tab,
+                        static_cast<void *>(d_units), static_cast<void *>(d_counter),
                         static_cast<void *>(d_rec), static_cast<void *>(d_frec),
                         static_cast<void *>(d_rec64), static_cast<void *>(d_fxrange),
                         static_cast<void *>(d_part),
@@ -161,7 +159,7 @@ bool scalar_only(const gsc_batch &b) {
 
 int occupancy(const gsc_batch &b, const Cfg &c) {
     if (is_fx(b)) return batch_fx_occupancy(c.R, scalar_only(b));
-    return is_plain(b) ? batch_plain_occupancy(c.R, c.tile, b.device)
+    return is_plain(b) ? batch_plain_occupancy(c.R)
                        : batch_mixed_occupancy(c.R, true, b.device);
 }
 
@@ -226,7 +224,7 @@ int fill_items(gsc_batch &b, const gsc_batch_item *items, int64_t count, bool ch
 // counts they imply.  Fills b.items[*].splits.
 int make_units(gsc_batch &b, const Cfg &c, int blocks, std::vector<BatchUnit> &units) {
     const int64_t ppb = static_cast<int64_t>(kBatchThreads) * c.R;
-    const int tile = is_plain(b) ? c.tile : mixed_tile(b);
+    const int tile = is_plain(b) ? kPlainGroupModes : mixed_tile(b);
     const double target = std::max(1.0, b.total_work / (static_cast<double>(blocks) * c.upb));
     units.clear();
     std::vector<double> cost;
@@ -407,8 +405,8 @@ int enqueue_tables(gsc_batch &b, cudaStream_t st) {
                                b.total_modes, reinterpret_cast<uint32_t *>(b.d_frec), b.d_fxrange,
                                b.range_flag, st);
     if (is_plain(b))
-        return batch_plain_tables(b.d_items, b.d_prefix, static_cast<int64_t>(b.items.size()),
-                                  b.total_modes, b.d_tab, b.d_rec, st);
+        return batch_plain_tables(b.d_items, static_cast<int64_t>(b.items.size()), b.total_modes,
+                                  b.d_rec, st);
     return batch_mixed_tables(b.d_items, b.d_prefix, static_cast<int64_t>(b.items.size()),
                               b.total_modes, b.d_frec, b.d_rec64, st);
 }
@@ -421,8 +419,7 @@ int enqueue_sum(gsc_batch &b, const Cfg &c, int blocks, int64_t n_units, cudaStr
                                b.d_counter, reinterpret_cast<const uint32_t *>(b.d_frec),
                                b.d_fxrange, st);
     if (is_plain(b))
-        return batch_plain_launch(c.R, c.tile, blocks, b.d_items, b.d_units, n_units, b.d_counter,
-                                  b.d_tab, b.d_rec, st);
+        return batch_plain_launch(c.R, blocks, b.d_items, b.d_units, n_units, b.d_counter, b.d_rec, st);
     return batch_mixed_launch(c.R, b.form == GSC_FORM_MIXED_F64PHASE, blocks, b.d_items, b.d_units,
                               n_units, b.d_counter, b.d_frec, b.d_rec64, st);
 }
@@ -460,7 +457,7 @@ std::vector<Cfg> candidates(const gsc_batch &b) {
     std::vector<Cfg> out;
     const int upbs[2] = {4, 16};
     if (is_plain(b)) {
-        const int rt[4][2] = {{2, 8}, {4, 8}, {4, 16}, {8, 8}};
+        const int rt[3][2] = {{2, 8}, {4, 8}, {8, 8}};
         for (auto &x : rt)
             for (int u : upbs) out.push_back(Cfg{x[0], x[1], u});
     } else {
@@ -585,7 +582,6 @@ int gsc_batch_create(const gsc_batch_item *items, int64_t count, const gsc_opts 
                         cudaMemcpyHostToDevice));
     const size_t M = static_cast<size_t>(b->total_modes);
     if (is_plain(*b)) {
-        GSC_TRY(dmalloc(&b->d_tab, M * kPlainTableBytesPerMode));
         GSC_TRY(dmalloc(reinterpret_cast<void **>(&b->d_rec), M * kPlainRecBytesPerMode));
     } else if (is_fx(*b)) {
         GSC_TRY(dmalloc(reinterpret_cast<void **>(&b->d_frec), M * kFxRecBytesPerMode));

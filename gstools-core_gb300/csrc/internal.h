@@ -242,7 +242,7 @@ int mixed_fx_run(DeviceCtx &ctx, const PlainArgs &a, int *range_flag, cudaStream
 // f64phase = false forwards to mixed_fx_run.
 int mixed_run(DeviceCtx &ctx, const PlainArgs &a, bool f64phase, cudaStream_t st);
 
-// Allocation-free scalar summator (plain.cu): per-mode tables in a fixed
+// Allocation-free scalar summator (plain.cu): mode records in a fixed
 // device array of kNoAllocModes modes; `device` must be current.
 constexpr int64_t kNoAllocModes = 1024;
 int plain_noalloc_run(int device, const PlainArgs &a, cudaStream_t st);
@@ -296,27 +296,25 @@ struct BatchUnit {
 };
 constexpr int kBatchThreads = 128;   // threads per block of the batch kernels
 
-// Per-mode tables of every item, one launch (plain.cu / mixed.cu).  mode_prefix
+// Mode records of every item, one launch (plain.cu / mixed.cu).  mode_prefix
 // has n_items + 1 entries (exclusive prefix sums of n_modes).
-int batch_plain_tables(const BatchItem *items, const int64_t *mode_prefix, int64_t n_items,
-                       int64_t total_modes, void *wtab, double *rec, cudaStream_t st);
+int batch_plain_tables(const BatchItem *items, int64_t n_items, int64_t total_modes, double *rec,
+                       cudaStream_t st);
 int batch_mixed_tables(const BatchItem *items, const int64_t *mode_prefix, int64_t n_items,
                        int64_t total_modes, float *rec, double *rec64, cudaStream_t st);
 // Persistent kernels fed from the work queue `units` through `counter`
-// (zero before the launch).  Shared-memory bytes and occupancy per config:
-size_t batch_plain_smem(int tile);
-int batch_plain_occupancy(int R, int tile, int device);
+// (zero before the launch), and their occupancy per config:
+int batch_plain_occupancy(int R);
 int batch_mixed_occupancy(int R, bool f64phase, int device);
 bool batch_plain_config_ok(int R, int tile);
 bool batch_mixed_config_ok(int R);
-int batch_plain_launch(int R, int tile, int blocks, const BatchItem *items,
-                       const BatchUnit *units, int64_t n_units, int *counter, const void *wtab,
-                       const double *rec, cudaStream_t st);
+int batch_plain_launch(int R, int blocks, const BatchItem *items, const BatchUnit *units,
+                       int64_t n_units, int *counter, const double *rec, cudaStream_t st);
 int batch_mixed_launch(int R, bool f64phase, int blocks, const BatchItem *items,
                        const BatchUnit *units, int64_t n_units, int *counter, const float *rec,
                        const double *rec64, cudaStream_t st);
-constexpr int64_t kPlainTableBytesPerMode = 256 * 16;   // W_j[a], a < 256, double2
-constexpr int64_t kPlainRecBytesPerMode = 12 * 8;
+constexpr int64_t kPlainRecBytesPerMode = 18 * 8;
+constexpr int kPlainGroupModes = 32;   // modes summed as integers of one scale: ranges start on a multiple
 constexpr int64_t kMixedRecBytesPerMode = 20 * 4;
 constexpr int64_t kMixedRec64BytesPerMode = 4 * 8;
 constexpr int64_t kFxRecBytesPerMode = 64 * 4;      // mixed_fx.cu mode record

@@ -1,30 +1,29 @@
 // plain.cu -- FP64 randomization-method summators for GB300 (sm_103a).
 //
-// Computes, in FP64 end to end,
+// Computes, to FP64 accuracy end to end,
 //   scalar   u[p]    = sum_j z1_j cos(k_j.x_p) + z2_j sin(k_j.x_p)
 //            (reference: src/field.rs:37-65)
 //   incompr  u[i, p] = sum_j w_ij (z1_j cos(k_j.x_p) + z2_j sin(k_j.x_p)),
 //            w_0j = 1 - k_0j k_0j/|k_j|^2, w_ij = -k_ij k_0j/|k_j|^2
 //            (reference: src/field.rs:97-182)
 //
-// Design.  GB300's FP64 pipe is narrow, so the kernel is built to spend as
-// few FP64 instructions per point*mode as possible while staying FP64
-// accurate:
-//  * phase k.x is formed exactly as the reference forms it:
+// Design.  GB300's FP64 pipe issues 2 lanes per clock and SM, so only what
+// needs its rounding stays on it; the rest runs on the integer pipes beside it:
+//  * phase k.x in FP64, formed exactly as the reference forms it:
 //    ((k0*x0 + k1*x1) + k2*x2), no FMA, so every phase has the reference's
-//    bits (src/field.rs:57, src/short_vec.rs:30-33);
-//  * sincos is table driven (Tang-style): phase = n*(2pi/M) + r with a
-//    two-constant Cody-Waite reduction (exact first step under FMA) and
-//    |r| <= pi/M, M = 256; e^{ir} by short Taylor polynomials (truncation
-//    below 5e-15), and the angle n*(2pi/M) folded into a per-mode table
-//    W_j[a] = (z1_j - i z2_j) e^{i 2 pi a/M}, so
-//    z1 cos(phase) + z2 sin(phase) = Re(W_j[n mod M] e^{ir})
-//    = Re W cos r - Im W sin r: 18 FP64 operations per point*mode for d=3;
-//  * per-mode tables live in global memory and are staged tile by tile into
-//    shared memory with cp.async double buffering; each thread keeps R
-//    points in registers, so one staged tile serves T*R points;
-//  * phases beyond |k.x| ~ 1e13 (where the one-step reduction would lose
-//    accuracy) take CUDA's sincos() for the whole tile (warp-uniform test);
+//    bits (src/field.rs:57, src/short_vec.rs:30-33): 2d - 1 instructions;
+//  * z1 cos + z2 sin = A cos(phase - beta), A = |z1 + i z2| and beta its
+//    angle, set up per mode (plain_rec_kernel); the phase becomes a 64-bit
+//    fraction of a turn and its cosine a 64-bit integer (fix64.cuh: 1.2e-16
+//    RMS), one integer multiply by A (scaled by the largest A of 32 modes, to
+//    2^-57 of it) and a 64-bit sum over those 32 modes, which is exact; one
+//    FP64 multiply-add per 32 modes adds it to the point's total.
+//    The FP64 polynomials, table products and sums that this replaces were 18
+//    FP64 instructions per point*mode for d = 3 (16 for d = 2); @@FIG@@
+//  * phases of 2^32 and more, and modes with a NaN or an infinity, take CUDA's
+//    sincos() and FP64 sums for that mode (the same test for a whole warp);
+//  * mode records (96 bytes) are staged 32 at a time into shared memory with
+//    cp.async double buffering; each thread keeps R points in registers;
 //  * when there are too few points to fill 152 SMs, the modes are split
 //    across blockIdx.y and the partial sums are added in split order by a
 //    second kernel (deterministic; no atomics).
@@ -36,25 +35,30 @@
 #include <mutex>
 #include <string>
 
+#include "fix64.cuh"
 #include "internal.h"
 
 namespace gsc {
 namespace {
 
-constexpr int kM = 256;                             // table angles per turn
-constexpr double kInvStep = 40.74366543152521;      // M / (2 pi)
-constexpr double kStepHi = 0.02454369260617026;     // fl(2 pi / M) = fl(pi)/128
-constexpr double kStepLo = 9.567553118338697e-19;   // fl(2 pi / M - kStepHi)
-constexpr double kRound = 6755399441055744.0;       // 1.5 * 2^52: x + kRound rounds x
-constexpr double kSafePhase = 1.0e13;               // table path bound on |k.x|
-constexpr int kRec = 12;                            // doubles per mode record
 constexpr int kThreads = 128;                       // threads per block
-constexpr int kTileModes = 8;                       // modes per staged tile
-constexpr int64_t kChunkModes = 16384;              // modes per table build
+constexpr int kGroup = kPlainGroupModes;            // modes per staged tile and integer sum
+constexpr int64_t kChunkModes = 1 << 20;            // modes per record build
 static_assert(kThreads == kBatchThreads, "batch units assume the plain block size");
+static_assert(kGroup == 32, "a warp builds the records of a group");
 
-// Mode record layout (doubles): k0 k1 k2 | sum|k| | z1 z2 | w0 w1 w2 | pad
-enum { R_K0 = 0, R_KABS = 3, R_Z1 = 4, R_Z2 = 5, R_W0 = 6 };
+// Mode record (8-byte words): what the sums read from shared memory, then the
+// FP64 weights of the exact path.
+//   k0 k1 | k2, |k| bound (FP32) | -beta + kCosOffset, A0 | A1 A2 | s0 s1 | s2 -
+//   z1 z2 | w0 w1 | w2 -
+// A_i = A w_i (A alone for the scalar field) as an integer of units s_i 2^-8
+// held in two words {high, low / 2}; s_i = 2^(e_i - 56), 2^(e_i) above every
+// |A_i| of the mode's group of 32.  The bound is infinite for a mode of the
+// exact path.
+constexpr int kRec = 18, kRecStaged = 12;
+enum { R_K0 = 0, R_K2 = 2, R_KABS = 3, R_BETA = 4, R_A0 = 5, R_S0 = 8, R_Z1 = 12, R_Z2 = 13, R_W0 = 14 };
+static_assert(kRec * 8 == kPlainRecBytesPerMode, "record layout");
+constexpr float kFastPhase = 4.29e9f;               // |k| |x| bound of the integer path, below 2^32
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
@@ -65,85 +69,130 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
 // ---------------------------------------------------------------------------
-// Per-mode tables: W_j[a] = (z1 - i z2) e^{i 2 pi a / M} and the mode record.
-// grid (nc), block (kM)
+// Mode records.  One warp per group of 32 modes, lane = mode (live: it exists);
+// all lanes call.  Everything but the last few FP64 operations is integer
+// arithmetic: an FP64 atan2 and hypot would be a chain of several microseconds
+// and less exact.
 // ---------------------------------------------------------------------------
-// Table row a (thread) and, for a == 0, the record of mode j.
-__device__ __forceinline__ void mode_entry(const double *__restrict__ cov, double z1j, double z2j,
-                                           int64_t dim, int64_t n_modes, int64_t j, int incompr,
-                                           int want_table, double2 *__restrict__ wrow,
-                                           double *__restrict__ r) {
-    const int a = threadIdx.x;
-    if (want_table) {
-        double s, c;
-        sincospi(a * (1.0 / (kM / 2)), &s, &c);       // angle 2 pi a / M
-        wrow[a] = make_double2(z1j * c + z2j * s, z1j * s - z2j * c);
-    }
-    if (a == 0) {
-        double k[3] = {0.0, 0.0, 0.0};
+__device__ __forceinline__ void rec_group(const double *__restrict__ cov, int64_t n_modes, int dim,
+                                          int64_t j, bool live, double z1, double z2, int incompr,
+                                          double *__restrict__ r, const CosTable *tab) {
+    double k[3] = {0.0, 0.0, 0.0}, w[3] = {0.0, 0.0, 0.0};
+    if (live)
         for (int d = 0; d < dim && d < 3; ++d) k[d] = cov[d * n_modes + j];
-        r[R_K0 + 0] = k[0];
-        r[R_K0 + 1] = k[1];
-        r[R_K0 + 2] = k[2];
-        r[R_KABS] = fabs(k[0]) + fabs(k[1]) + fabs(k[2]);
-        r[R_Z1] = z1j;
-        r[R_Z2] = z2j;
-        double w0 = 0.0, w1 = 0.0, w2 = 0.0;
-        if (incompr) {
-            // src/field.rs:138: k_2 = k0 / k.k, ShortVec::dot order, no FMA
-            double kk = 0.0;
-            for (int d = 0; d < dim; ++d) kk = __dadd_rn(kk, __dmul_rn(k[d], k[d]));
-            const double k_2 = __ddiv_rn(k[0], kk);
-            w0 = __dadd_rn(1.0, -__dmul_rn(k[0], k_2));          // :148
-            w1 = -__dmul_rn(k[1], k_2);                            // :150-152
-            w2 = -__dmul_rn(k[2], k_2);
+    bool regular = isfinite(z1) && isfinite(z2) && isfinite(k[0]) && isfinite(k[1]) && isfinite(k[2]);
+    if (incompr) {
+        // src/field.rs:138: k_2 = k0 / k.k, ShortVec::dot order, no FMA
+        double kk = 0.0;
+        for (int d = 0; d < dim; ++d) kk = __dadd_rn(kk, __dmul_rn(k[d], k[d]));
+        const double k_2 = __ddiv_rn(k[0], kk);
+        w[0] = __dadd_rn(1.0, -__dmul_rn(k[0], k_2));          // :148
+        w[1] = -__dmul_rn(k[1], k_2);                            // :150-152
+        w[2] = -__dmul_rn(k[2], k_2);
+        regular = regular && isfinite(w[0]) && isfinite(w[1]) && isfinite(w[2]);
+    }
+    // z1 + i z2 = A e^{i beta}: a first angle in FP32, its cosine and sine in
+    // 64 bits, then the remaining rotation d (1e-7 rad) from the cross product
+    uint64_t beta = 0;
+    double amp = 0.0;                                            // A 2^-ez
+    int ez = 0;
+    const double zm = fmax(fabs(z1), fabs(z2));
+    if (regular && zm > 0.0) {
+        frexp(zm, &ez);
+        const double y1 = ldexp(z1, -ez), y2 = ldexp(z2, -ez);
+        const float t = atan2f(static_cast<float>(y2), static_cast<float>(y1)) * 0.15915494f;   // turns
+        beta = static_cast<uint64_t>(__float2ll_rn(t * 1099511627776.0f)) << 24;
+        const int64_t f1 = __double2ll_rn(y1 * 0x1p62), f2 = __double2ll_rn(y2 * 0x1p62);
+        const int64_t c = cos_fixed(beta + kCosOffset, tab);
+        const int64_t s = cos_fixed(beta - (uint64_t(1) << 62) + kCosOffset, tab);
+        const double along = static_cast<double>(__mul64hi(f1, c) + __mul64hi(f2, s));    // units 2^-60
+        const double across = static_cast<double>(__mul64hi(f2, c) - __mul64hi(f1, s));
+        const double d = across / along;
+        amp = fma(along, 0.5 * d * d, along) * 0x1p-60;
+        beta += static_cast<uint64_t>(__double2ll_rn(d * 2.935890503282001e18));          // 2^64 / 2 pi
+    }
+    const int nout = incompr ? dim : 1;
+    double a[3] = {incompr ? amp * w[0] : amp, amp * w[1], amp * w[2]};
+    double scale[3] = {0.0, 0.0, 0.0};
+    long long fix[3] = {0, 0, 0};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        if (i >= nout) continue;
+        int e = -100000;
+        if (regular && a[i] != 0.0) {
+            frexp(a[i], &e);
+            e += ez;
         }
-        r[R_W0 + 0] = w0;
-        r[R_W0 + 1] = w1;
-        r[R_W0 + 2] = w2;
-        r[9] = r[10] = r[11] = 0.0;
+        const int eg = __reduce_max_sync(0xffffffffu, e);
+        if (eg == -100000) continue;                             // all zero: scale 0
+        if (eg < -900 || eg > 900) {
+            regular = false;
+            continue;
+        }
+        if (regular) fix[i] = __double2ll_rn(ldexp(a[i], ez - eg + 58));
+        scale[i] = ldexp(1.0, eg - 56);
     }
+    if (!live) return;
+    r[R_K0] = k[0];
+    r[R_K0 + 1] = k[1];
+    r[R_K2] = k[2];
+    const float kabs = regular ? __double2float_ru(fabs(k[0]) + fabs(k[1]) + fabs(k[2]))
+                               : __int_as_float(0x7f800000);
+    r[R_KABS] = __hiloint2double(0, __float_as_int(kabs));
+    r[R_BETA] = __longlong_as_double(static_cast<long long>(kCosOffset - beta));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        r[R_A0 + i] = __hiloint2double(static_cast<int>(static_cast<uint32_t>(fix[i]) >> 1),
+                                       static_cast<int>(fix[i] >> 32));
+        r[R_S0 + i] = scale[i];
+        r[R_W0 + i] = w[i];
+    }
+    r[R_S0 + 3] = 0.0;
+    r[R_Z1] = z1;
+    r[R_Z2] = z2;
+    r[R_W0 + 3] = 0.0;
 }
 
-__global__ void __launch_bounds__(kM)
-mode_table_kernel(const double *__restrict__ cov, const double *__restrict__ z1,
-                  const double *__restrict__ z2, int64_t dim, int64_t n_modes, int64_t j0,
-                  int incompr, int want_table, double2 *__restrict__ wtab,
-                  double *__restrict__ rec, const int *__restrict__ run_if) {
+// Records of modes [j0, j0 + nc); grid ceil(nc / kThreads), j0 a multiple of 32.
+__global__ void __launch_bounds__(kThreads)
+plain_rec_kernel(const double *__restrict__ cov, const double *__restrict__ z1,
+                 const double *__restrict__ z2, int dim, int64_t n_modes, int64_t j0, int64_t nc,
+                 int incompr, double *__restrict__ rec, const int *__restrict__ run_if) {
     if (run_if && *run_if == 0) return;      // a predicated launch that is not wanted
-    const int64_t jl = blockIdx.x;
-    const int64_t j = j0 + jl;
-    mode_entry(cov, z1[j], z2[j], dim, n_modes, j, incompr, want_table, wtab + jl * kM,
-               rec + jl * kRec);
+    __shared__ CosTable tab;
+    const int64_t jl = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x, j = j0 + jl;
+    const bool live = jl < nc;
+    const double a = live ? z1[j] : 0.0, b = live ? z2[j] : 0.0;
+    fill_cos_table(&tab, threadIdx.x, kThreads);
+    __syncthreads();
+    rec_group(cov, n_modes, dim, j, live, a, b, incompr, rec + jl * kRec, &tab);
 }
 
-// item owning global row g: the last i with prefix[i] <= g
-__device__ __forceinline__ int64_t owner_of(const int64_t *__restrict__ prefix, int64_t n,
-                                            int64_t g) {
-    int64_t lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int64_t mid = (lo + hi + 1) >> 1;
-        if (prefix[mid] <= g) lo = mid; else hi = mid - 1;
+// Records of every item of a batch: the warps of column blockIdx.y walk the
+// groups of item blockIdx.y.  The Fourier factor, where present, multiplies z1
+// and z2 first.
+__global__ void __launch_bounds__(kThreads)
+batch_rec_kernel(const BatchItem *__restrict__ items, int64_t n_items, double *__restrict__ rec) {
+    __shared__ CosTable tab;
+    fill_cos_table(&tab, threadIdx.x, kThreads);
+    __syncthreads();
+    for (int64_t i = blockIdx.y; i < n_items; i += gridDim.y) {
+        const BatchItem &it = items[i];
+        const int64_t groups = (it.n_modes + kGroup - 1) / kGroup;
+        for (int64_t g = static_cast<int64_t>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5);
+             g < groups; g += static_cast<int64_t>(gridDim.x) * (kThreads / 32)) {
+            const int64_t j = g * kGroup + (threadIdx.x & 31);
+            const bool live = j < it.n_modes;
+            double a = live ? it.z1[j] : 0.0, b = live ? it.z2[j] : 0.0;
+            if (live && it.sf) {
+                const double f = it.sf[j];
+                a = __dmul_rn(f, a);
+                b = __dmul_rn(f, b);
+            }
+            rec_group(it.cov, it.n_modes, it.dim, j, live, a, b, it.incompr,
+                      rec + (it.mode_off + j) * kRec, &tab);
+        }
     }
-    return lo;
-}
-
-// Tables of every item of a batch: grid (total modes), block (kM).  The
-// Fourier factor, where present, multiplies z1 and z2 first.
-__global__ void __launch_bounds__(kM)
-batch_table_kernel(const BatchItem *__restrict__ items, const int64_t *__restrict__ prefix,
-                   int64_t n_items, double2 *__restrict__ wtab, double *__restrict__ rec) {
-    const int64_t g = blockIdx.x;
-    const BatchItem &it = items[owner_of(prefix, n_items, g)];
-    const int64_t j = g - it.mode_off;
-    double z1j = it.z1[j], z2j = it.z2[j];
-    if (it.sf) {
-        const double f = it.sf[j];
-        z1j = __dmul_rn(f, z1j);
-        z2j = __dmul_rn(f, z2j);
-    }
-    mode_entry(it.cov, z1j, z2j, it.dim, it.n_modes, j, it.incompr, 1, wtab + g * kM,
-               rec + g * kRec);
 }
 
 // phase = k.x in the reference's order (ndarray dot on strided columns)
@@ -155,121 +204,132 @@ __device__ __forceinline__ double phase_of(const double *k, const double *x) {
     return ph;
 }
 
-// z1 cos(ph) + z2 sin(ph) through the mode's angle table (see file header).
-__device__ __forceinline__ double table_term(double ph, const double2 *__restrict__ tab) {
-    const double s = fma(ph, kInvStep, kRound);
-    const double n = s - kRound;
-    const int a = __double2loint(s) & (kM - 1);
-    double r = fma(-n, kStepHi, ph);          // exact
-    r = fma(-n, kStepLo, r);
-    const double r2 = r * r;
-    const double cr = fma(r2, fma(r2, 1.0 / 24.0, -0.5), 1.0);
-    const double sr = fma(r * r2, fma(r2, 1.0 / 120.0, -1.0 / 6.0), r);
-    const double2 w = tab[a];
-    return fma(w.x, cr, -(w.y * sr));
-}
+struct PlainSmem {
+    CosTable tab;
+    __align__(16) double rec[2][kGroup * kRecStaged];
+};
 
 // ---------------------------------------------------------------------------
 // One block's work: the kThreads*R points starting at p_first (thread t owns
-// p_first + t + r*kThreads), modes [jb, je) of the staged tables `wtab`,
-// `rec` (indices relative to them), TILE modes per staged tile.  The sums are
-// written (accumulate=0) or added (accumulate=1) at dst + i*sd + p*sp.
-// Shared memory: 2 * TILE * (kM*16 [table] + kRec*8) bytes at `smem`.
+// p_first + t + r*kThreads), modes [jb, je) of the records `rec` (indices
+// relative to them; jb a multiple of kGroup).  The sums are written
+// (accumulate=0) or added (accumulate=1) at dst + i*sd + p*sp.  sm.tab is
+// filled by the caller (not read by LIBM, CUDA's sincos() for every mode).
 // ---------------------------------------------------------------------------
-template <int D, int R, bool INC, bool LIBM, int TILE>
+template <int D, int R, bool INC, bool LIBM>
 __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int64_t P,
-                                            int64_t p_first, const double2 *__restrict__ wtab,
-                                            const double *__restrict__ rec, int64_t jb,
-                                            int64_t je, int accumulate, double *__restrict__ dst,
-                                            int64_t sd, int64_t sp, unsigned char *smem) {
+                                            int64_t p_first, const double *__restrict__ rec,
+                                            int64_t jb, int64_t je, int accumulate,
+                                            double *__restrict__ dst, int64_t sd, int64_t sp,
+                                            PlainSmem &sm) {
     constexpr int NOUT = INC ? D : 1;
-    constexpr int TAB_BYTES = LIBM ? 0 : TILE * kM * 16;
-    constexpr int REC_BYTES = TILE * kRec * 8;
-    constexpr int STAGE = TAB_BYTES + REC_BYTES;
-
     const int tid = threadIdx.x;
     const int64_t p0 = p_first + tid;
+
+    auto stage_tile = [&](int buf, int64_t t0) {
+        const int chunks = static_cast<int>(min(static_cast<int64_t>(kGroup), je - t0)) * (kRecStaged / 2);
+        const double *src = rec + t0 * kRec;
+        for (int c = tid; c < chunks; c += kThreads) {
+            const int m = c / (kRecStaged / 2), q = c - m * (kRecStaged / 2);
+            cp_async16(&sm.rec[buf][m * kRecStaged + 2 * q], src + m * kRec + 2 * q);
+        }
+        cp_async_commit();
+    };
+    if (jb < je) stage_tile(0, jb);
 
     double x[R][D];
     double acc[R][NOUT];
     double xabs = 0.0;
+    bool bad[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int64_t p = p0 + r * kThreads;
         double s = 0.0;
+        bad[r] = false;
 #pragma unroll
         for (int d = 0; d < D; ++d) {
             x[r][d] = p < P ? pos[d * P + p] : 0.0;
+            bad[r] = bad[r] || isnan(x[r][d]);
             s += fabs(x[r][d]);
         }
         xabs = fmax(xabs, s);
 #pragma unroll
         for (int i = 0; i < NOUT; ++i) acc[r][i] = 0.0;
     }
-    // warp-uniform bound on |x| for the table-path range test
+    // warp-uniform bound on |x| for the range test (NaN coordinates do not
+    // count: their points end as NaN)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) xabs = fmax(xabs, __shfl_xor_sync(0xffffffffu, xabs, o));
+    const float xbound = __double2float_ru(xabs);
 
-    auto stage_tile = [&](int buf, int64_t t0) {
-        const int tm = static_cast<int>(min(static_cast<int64_t>(TILE), je - t0));
-        unsigned char *base = smem + buf * STAGE;
-        if (!LIBM) {
-            const int chunks = tm * kM;                      // 16-byte chunks
-            const double2 *src = wtab + (t0)*kM;
-            for (int c = tid; c < chunks; c += kThreads) cp_async16(base + c * 16, src + c);
-        }
-        const int rchunks = tm * kRec / 2;
-        const double *rsrc = rec + t0 * kRec;
-        for (int c = tid; c < rchunks; c += kThreads)
-            cp_async16(base + TAB_BYTES + c * 16, rsrc + 2 * c);
-        cp_async_commit();
-    };
-
-    if (jb < je) stage_tile(0, jb);
     int buf = 0;
-    for (int64_t t0 = jb; t0 < je; t0 += TILE, buf ^= 1) {
-        const int tm = static_cast<int>(min(static_cast<int64_t>(TILE), je - t0));
-        if (t0 + TILE < je) {
-            stage_tile(buf ^ 1, t0 + TILE);
+    for (int64_t t0 = jb; t0 < je; t0 += kGroup, buf ^= 1) {
+        const int tm = static_cast<int>(min(static_cast<int64_t>(kGroup), je - t0));
+        if (t0 + kGroup < je) {
+            stage_tile(buf ^ 1, t0 + kGroup);
             cp_async_wait<1>();
         } else {
             cp_async_wait<0>();
         }
         __syncthreads();
-        const unsigned char *base = smem + buf * STAGE;
-        const double2 *tab = reinterpret_cast<const double2 *>(base);
-        const double *rc = reinterpret_cast<const double *>(base + TAB_BYTES);
+        const double *rc = sm.rec[buf];
+        // sums over the group in units s_i 2^-56 ...; the truncated products of
+        // a term leave out two units on average
+        long long sum[R][NOUT];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int i = 0; i < NOUT; ++i) sum[r][i] = 2 * tm;
+#pragma unroll 1
         for (int m = 0; m < tm; ++m) {
-            const double *mr = rc + m * kRec;
-            double k[3] = {mr[R_K0], mr[R_K0 + 1], mr[R_K0 + 2]};
-            double w[3] = {mr[R_W0], mr[R_W0 + 1], mr[R_W0 + 2]};
-            const bool table_ok = !LIBM && (mr[R_KABS] * xabs < kSafePhase);
-            if (table_ok) {
-                const double2 *mt = tab + m * kM;
+            const double2 *mr = reinterpret_cast<const double2 *>(rc + m * kRecStaged);
+            const double2 q0 = mr[0], q1 = mr[1];
+            const double k[3] = {q0.x, q0.y, q1.x};
+            const float kb = __int_as_float(__double2loint(q1.y));
+            if (!LIBM && kb * xbound < kFastPhase) {
+                const double2 q2 = mr[2];
+                const uint64_t beta = static_cast<uint64_t>(__double_as_longlong(q2.x));
+                double av[3] = {q2.y, 0.0, 0.0};
+                if (INC) {
+                    const double2 q3 = mr[3];
+                    av[1] = q3.x;
+                    av[2] = q3.y;
+                }
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
-                    const double z12 = table_term(phase_of<D>(k, x[r]), mt);
-                    if (INC) {
+                    const int64_t c = cos_fixed(turn_fraction(phase_of<D>(k, x[r])) + beta, &sm.tab);
+                    const int32_t ch = static_cast<int32_t>(c >> 32);
+                    const int32_t c0 = static_cast<int32_t>(static_cast<uint32_t>(c) >> 1);
 #pragma unroll
-                        for (int i = 0; i < NOUT; ++i) acc[r][i] = fma(w[i], z12, acc[r][i]);
-                    } else {
-                        acc[r][0] = __dadd_rn(acc[r][0], z12);
+                    for (int i = 0; i < NOUT; ++i) {
+                        const int32_t ah = __double2loint(av[i]), a0 = __double2hiint(av[i]);
+                        sum[r][i] += static_cast<int64_t>(ah) * ch;
+                        sum[r][i] += static_cast<int64_t>(__mulhi(ah, c0) + __mulhi(a0, ch)) << 1;
                     }
                 }
             } else {
-                const double z1 = mr[R_Z1], z2 = mr[R_Z2];
+                const double *ex = rec + (t0 + m) * kRec;
+                const double z1 = ex[R_Z1], z2 = ex[R_Z2];
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     double sn, cs;
                     sincos(phase_of<D>(k, x[r]), &sn, &cs);
                     const double z12 = __dadd_rn(__dmul_rn(z1, cs), __dmul_rn(z2, sn));
-                    if (INC) {
 #pragma unroll
-                        for (int i = 0; i < NOUT; ++i) acc[r][i] = fma(w[i], z12, acc[r][i]);
-                    } else {
-                        acc[r][0] = __dadd_rn(acc[r][0], z12);
+                    for (int i = 0; i < NOUT; ++i) {
+                        if (INC) acc[r][i] = fma(ex[R_W0 + i], z12, acc[r][i]);
+                        else acc[r][i] = __dadd_rn(acc[r][i], z12);
+                        if (!LIBM) sum[r][i] -= 2;
                     }
                 }
+            }
+        }
+        if (!LIBM) {
+#pragma unroll
+            for (int i = 0; i < NOUT; ++i) {
+                const double s = rc[R_S0 + i];
+#pragma unroll
+                for (int r = 0; r < R; ++r) acc[r][i] = fma(static_cast<double>(sum[r][i]), s, acc[r][i]);
             }
         }
         __syncthreads();   // buffer `buf` is refilled two tiles later
@@ -281,8 +341,10 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
         if (p >= P) continue;
 #pragma unroll
         for (int i = 0; i < NOUT; ++i) {
+            double v = acc[r][i];
+            if (bad[r] && jb < je) v = __longlong_as_double(0x7ff8000000000000ll);
             double *o = dst + i * sd + p * sp;
-            *o = accumulate ? *o + acc[r][i] : acc[r][i];
+            *o = accumulate ? *o + v : v;
         }
     }
 }
@@ -295,17 +357,17 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
 // ---------------------------------------------------------------------------
 template <int D, int R, bool INC, bool LIBM>
 __global__ void __launch_bounds__(kThreads)
-plain_kernel(const double *__restrict__ pos, int64_t P, const double2 *__restrict__ wtab,
-             const double *__restrict__ rec, int64_t nc, int64_t mps, int accumulate,
-             double *__restrict__ dst, int64_t sd, int64_t sp, int64_t split_stride,
-             const int *__restrict__ run_if) {
+plain_kernel(const double *__restrict__ pos, int64_t P, const double *__restrict__ rec, int64_t nc,
+             int64_t mps, int accumulate, double *__restrict__ dst, int64_t sd, int64_t sp,
+             int64_t split_stride, const int *__restrict__ run_if) {
     if (run_if && *run_if == 0) return;      // a predicated launch that is not wanted
-    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ PlainSmem sm;
+    if (!LIBM) fill_cos_table(&sm.tab, threadIdx.x, kThreads);   // read after the first tile's barrier
     const int64_t jb = static_cast<int64_t>(blockIdx.y) * mps;
     const int64_t je = min(nc, jb + mps);
-    plain_block<D, R, INC, LIBM, kTileModes>(
-        pos, P, static_cast<int64_t>(blockIdx.x) * (kThreads * R), wtab, rec, jb, je, accumulate,
-        dst + static_cast<int64_t>(blockIdx.y) * split_stride, sd, sp, smem);
+    plain_block<D, R, INC, LIBM>(pos, P, static_cast<int64_t>(blockIdx.x) * (kThreads * R), rec, jb, je,
+                                 accumulate, dst + static_cast<int64_t>(blockIdx.y) * split_stride, sd,
+                                 sp, sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -314,13 +376,13 @@ plain_kernel(const double *__restrict__ pos, int64_t P, const double2 *__restric
 // of one item and one of its mode ranges; its sums go to the item's output,
 // or to its split slot when the item's modes are split.
 // ---------------------------------------------------------------------------
-template <int R, int TILE>
+template <int R>
 __global__ void __launch_bounds__(kThreads)
 batch_plain_kernel(const BatchItem *__restrict__ items, const BatchUnit *__restrict__ units,
-                   int64_t n_units, int *__restrict__ counter, const double2 *__restrict__ wtab,
-                   const double *__restrict__ rec) {
-    extern __shared__ __align__(16) unsigned char smem[];
+                   int64_t n_units, int *__restrict__ counter, const double *__restrict__ rec) {
+    __shared__ PlainSmem sm;
     __shared__ int s_unit;
+    fill_cos_table(&sm.tab, threadIdx.x, kThreads);
     for (;;) {
         __syncthreads();                     // s_unit of the previous unit is consumed
         if (threadIdx.x == 0) s_unit = atomicAdd(counter, 1);
@@ -332,28 +394,22 @@ batch_plain_kernel(const BatchItem *__restrict__ items, const BatchUnit *__restr
         const int64_t P = it.n_points;
         const int64_t nout = it.incompr ? it.dim : 1;
         double *dst = it.splits > 1 ? it.part + static_cast<int64_t>(w.split) * nout * P : it.out;
-        const double2 *wt = wtab + it.mode_off * kM;
         const double *rc = rec + it.mode_off * kRec;
         switch (it.dim * 2 + it.incompr) {
             case 2:
-                plain_block<1, R, false, false, TILE>(it.pos, P, w.p_first, wt, rc, w.jb, w.je, 0,
-                                                      dst, P, 1, smem);
+                plain_block<1, R, false, false>(it.pos, P, w.p_first, rc, w.jb, w.je, 0, dst, P, 1, sm);
                 break;
             case 4:
-                plain_block<2, R, false, false, TILE>(it.pos, P, w.p_first, wt, rc, w.jb, w.je, 0,
-                                                      dst, P, 1, smem);
+                plain_block<2, R, false, false>(it.pos, P, w.p_first, rc, w.jb, w.je, 0, dst, P, 1, sm);
                 break;
             case 5:
-                plain_block<2, R, true, false, TILE>(it.pos, P, w.p_first, wt, rc, w.jb, w.je, 0,
-                                                     dst, P, 1, smem);
+                plain_block<2, R, true, false>(it.pos, P, w.p_first, rc, w.jb, w.je, 0, dst, P, 1, sm);
                 break;
             case 6:
-                plain_block<3, R, false, false, TILE>(it.pos, P, w.p_first, wt, rc, w.jb, w.je, 0,
-                                                      dst, P, 1, smem);
+                plain_block<3, R, false, false>(it.pos, P, w.p_first, rc, w.jb, w.je, 0, dst, P, 1, sm);
                 break;
             case 7:
-                plain_block<3, R, true, false, TILE>(it.pos, P, w.p_first, wt, rc, w.jb, w.je, 0,
-                                                     dst, P, 1, smem);
+                plain_block<3, R, true, false>(it.pos, P, w.p_first, rc, w.jb, w.je, 0, dst, P, 1, sm);
                 break;
             default:
                 break;                       // rejected on the host
@@ -393,37 +449,82 @@ __global__ void generic_kernel(const double *__restrict__ cov, const double *__r
     out[p * sp] = sum;
 }
 
-template <int D, int R, bool INC, bool LIBM>
-int launch_main(dim3 grid, size_t smem, cudaStream_t st, const double *pos, int64_t P,
-                const double2 *wtab, const double *rec, int64_t nc, int64_t mps, int accumulate,
-                double *dst, int64_t sd, int64_t sp, int64_t split_stride, const int *run_if) {
-    auto fn = plain_kernel<D, R, INC, LIBM>;
-    GSC_TRY(smem_attr(reinterpret_cast<const void *>(fn), smem));   // once per device
-    fn<<<grid, kThreads, smem, st>>>(pos, P, wtab, rec, nc, mps, accumulate, dst, sd, sp,
-                                     split_stride, run_if);
-    GSC_CUDA(cudaGetLastError());
-    return GSC_OK;
-}
+// where a plain launch reads and writes; modes [0, nc) of rec in splits of mps
+struct PlainLaunch {
+    const double *pos;
+    int64_t P;
+    const double *rec;
+    int64_t nc, mps;
+    int accumulate;
+    double *dst;
+    int64_t sd, sp, split_stride;
+    const int *run_if;
+};
 
 template <int R, bool INC, bool LIBM>
-int dispatch_dim(int64_t dim, dim3 grid, size_t smem, cudaStream_t st, const double *pos,
-                 int64_t P, const double2 *wtab, const double *rec, int64_t nc, int64_t mps,
-                 int accumulate, double *dst, int64_t sd, int64_t sp, int64_t split_stride,
-                 const int *run_if = nullptr) {
-    switch (dim) {
-        case 1:
-            if (!INC)
-                return launch_main<1, R, INC, LIBM>(grid, smem, st, pos, P, wtab, rec, nc, mps,
-                                                    accumulate, dst, sd, sp, split_stride, run_if);
-            break;
-        case 2:
-            return launch_main<2, R, INC, LIBM>(grid, smem, st, pos, P, wtab, rec, nc, mps,
-                                                accumulate, dst, sd, sp, split_stride, run_if);
-        case 3:
-            return launch_main<3, R, INC, LIBM>(grid, smem, st, pos, P, wtab, rec, nc, mps,
-                                                accumulate, dst, sd, sp, split_stride, run_if);
+int dispatch_dim(int64_t dim, dim3 grid, cudaStream_t st, const PlainLaunch &l) {
+    auto launch = [&](auto fn) -> int {
+        fn<<<grid, kThreads, 0, st>>>(l.pos, l.P, l.rec, l.nc, l.mps, l.accumulate, l.dst, l.sd, l.sp,
+                                      l.split_stride, l.run_if);
+        GSC_CUDA(cudaGetLastError());
+        return GSC_OK;
+    };
+    if constexpr (!INC) {
+        if (dim == 1) return launch(plain_kernel<1, R, INC, LIBM>);
     }
+    if (dim == 2) return launch(plain_kernel<2, R, INC, LIBM>);
+    if (dim == 3) return launch(plain_kernel<3, R, INC, LIBM>);
     return set_error(GSC_ERR_DIM, "unsupported dimension for the plain kernel");
+}
+
+int dispatch_plain(int R, bool incompr, bool libm, int64_t dim, dim3 grid, cudaStream_t st,
+                   const PlainLaunch &l) {
+    if (libm)     // one launch shape: this form is a check on the others, not a fast path
+        return incompr ? dispatch_dim<4, true, true>(dim, grid, st, l)
+                       : dispatch_dim<4, false, true>(dim, grid, st, l);
+    if (R == 1)
+        return incompr ? dispatch_dim<1, true, false>(dim, grid, st, l)
+                       : dispatch_dim<1, false, false>(dim, grid, st, l);
+    if (R == 2)
+        return incompr ? dispatch_dim<2, true, false>(dim, grid, st, l)
+                       : dispatch_dim<2, false, false>(dim, grid, st, l);
+    return incompr ? dispatch_dim<4, true, false>(dim, grid, st, l)
+                   : dispatch_dim<4, false, false>(dim, grid, st, l);
+}
+
+// Launch shape: points per thread R and mode splits S (of mps modes, a
+// multiple of the group of 32), by the time of the busiest SM: its blocks'
+// point*modes, a fixed cost per block, and what the partial sums cost.
+struct PlainShape {
+    int R;
+    int64_t bx, S, mps;
+};
+PlainShape plain_shape(int64_t P, int64_t chunk, int64_t dim, int64_t nout, int sms, bool libm) {
+    PlainShape best{4, (P + 4 * kThreads - 1) / (4 * kThreads), 1, (chunk + kGroup - 1) / kGroup * kGroup};
+    double best_cost = 1e300;
+    // clocks a warp holds its quarter of the SM per point*mode: 34 for each
+    // FP64 instruction of a phase and half of the integer work beside it
+    const double pm = libm ? 2000.0 : std::max(68.0 * (2.0 * dim - 1.0), 130.0);
+    for (int R : {4, 2, 1}) {
+        if (libm && R != 4) continue;
+        const int64_t bx = (P + kThreads * R - 1) / (kThreads * R);
+        const int64_t groups = std::max<int64_t>(1, (chunk + kGroup - 1) / kGroup);
+        for (int64_t per = groups; per >= 1; --per) {
+            // only the group counts that some split count needs
+            const int64_t S = (groups + per - 1) / per;
+            if (S > 64) break;
+            if (per > 1 && (groups + per - 2) / (per - 1) == S) continue;   // a smaller share, same S
+            const double on_sm = std::ceil(static_cast<double>(bx) * S / sms);
+            double cost = on_sm * (per * kGroup * R * pm + 1500.0);
+            if (S > 1) cost += 4000.0 + static_cast<double>(S) * nout * P * 8.0 / 2000.0;
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = PlainShape{R, bx, S, per * kGroup};
+            }
+        }
+    }
+    if (chunk == 0) best.S = 1;
+    return best;
 }
 
 int sm_count(int device) {
@@ -551,74 +652,55 @@ int plain_run(DeviceCtx &ctx, const PlainArgs &a, cudaStream_t st) {
         return set_error(GSC_ERR_DIM, "Only two- and three-dimensional problems are supported.");
 
     // ---- launch geometry ---------------------------------------------------
-    const int64_t pts_per_block = static_cast<int64_t>(kThreads) * R;
-    const int64_t bx = (P + pts_per_block - 1) / pts_per_block;
-    if (bx > 0x7fffffff) return set_error(GSC_ERR_INVALID, "too many points for one launch");
     const int64_t chunk = std::min<int64_t>(N, kChunkModes);
-    const int64_t want_blocks = static_cast<int64_t>(sm_count(ctx.device)) * 6;
-    int64_t S = std::max<int64_t>(1, (want_blocks + bx - 1) / bx);
-    S = std::min<int64_t>(S, std::max<int64_t>(1, chunk / (2 * kTileModes)));
-    S = std::min<int64_t>(S, 64);
-    int64_t mps = chunk > 0 ? (chunk + S - 1) / S : 0;
-    mps = (mps + kTileModes - 1) / kTileModes * kTileModes;
-    if (mps > 0) S = std::max<int64_t>(1, (chunk + mps - 1) / mps);
-    if (N == 0) S = 1;
+    const PlainShape shp = plain_shape(P, chunk, dim, nout, sm_count(ctx.device), libm);
+    const int64_t S = shp.S;
+    if (shp.bx > 0x7fffffff) return set_error(GSC_ERR_INVALID, "too many points for one launch");
 
-    // ---- scratch: tables of one chunk, mode records, split partials --------
-    const size_t tab_bytes = libm ? 0 : static_cast<size_t>(chunk) * kM * sizeof(double2);
-    const size_t rec_bytes = static_cast<size_t>(chunk) * kRec * sizeof(double);
+    // ---- scratch: mode records of one chunk, split partials ------------------
+    const size_t rec_bytes = static_cast<size_t>(chunk) * kPlainRecBytesPerMode;
     const size_t part_bytes = S > 1 ? static_cast<size_t>(S) * nout * P * sizeof(double) : 0;
-    const size_t off_rec = (tab_bytes + 255) / 256 * 256;
-    const size_t off_part = off_rec + (rec_bytes + 255) / 256 * 256;
+    const size_t off_part = (rec_bytes + 255) / 256 * 256;
     GSC_TRY(ensure_dev(ctx, ctx.scratch, off_part + part_bytes + 256));
     GSC_CUDA(cudaStreamWaitEvent(st, ctx.scratch_ready, 0));
     unsigned char *sbase = static_cast<unsigned char *>(ctx.scratch.ptr);
-    double2 *wtab = reinterpret_cast<double2 *>(sbase);
-    double *rec = reinterpret_cast<double *>(sbase + off_rec);
+    double *rec = reinterpret_cast<double *>(sbase);
     double *part = reinterpret_cast<double *>(sbase + off_part);
 
-    double *dst = S > 1 ? part : a.out;
-    const int64_t sd = S > 1 ? P : a.out_sd;
-    const int64_t sp = S > 1 ? 1 : a.out_sp;
-    const int64_t split_stride = S > 1 ? nout * P : 0;
-    const size_t smem = 2 * ((libm ? 0 : kTileModes * kM * 16) + kTileModes * kRec * 8);
-    const dim3 grid(static_cast<unsigned>(bx), static_cast<unsigned>(S));
+    PlainLaunch l{};
+    l.pos = a.pos;
+    l.P = P;
+    l.rec = rec;
+    l.dst = S > 1 ? part : a.out;
+    l.sd = S > 1 ? P : a.out_sd;
+    l.sp = S > 1 ? 1 : a.out_sp;
+    l.split_stride = S > 1 ? nout * P : 0;
+    l.run_if = a.run_if;
 
     int64_t j0 = 0;
-    int first = 1;
     do {
         const int64_t nc = std::min<int64_t>(N - j0, kChunkModes);
         if (nc > 0) {
             TimedLaunch tl(st);
             tl.begin(K_MODE_TABLE);
-            mode_table_kernel<<<static_cast<unsigned>(nc), kM, 0, st>>>(
-                a.cov, a.z1, a.z2, dim, N, j0, a.incompr ? 1 : 0, libm ? 0 : 1, wtab, rec, a.run_if);
+            plain_rec_kernel<<<static_cast<unsigned>((nc + kThreads - 1) / kThreads), kThreads, 0, st>>>(
+                a.cov, a.z1, a.z2, static_cast<int>(dim), N, j0, nc, a.incompr ? 1 : 0, rec, a.run_if);
             tl.end();
             GSC_CUDA(cudaGetLastError());
         }
-        const int64_t mps_c = nc > 0 ? std::min<int64_t>(mps, nc) : 0;
-        const dim3 g(grid.x, static_cast<unsigned>(
-                                 nc > 0 ? std::min<int64_t>(S, (nc + mps_c - 1) / mps_c) : 1));
+        l.nc = nc;
+        l.mps = shp.mps;
+        l.accumulate = j0 > 0;
         // on later chunks, splits past the end of a short chunk are not
         // launched and keep their sums
-        const dim3 gl = first ? grid : g;
+        const int64_t s_used = (j0 == 0 || nc == 0) ? S : std::min<int64_t>(S, (nc + l.mps - 1) / l.mps);
         TimedLaunch tl(st);
         tl.begin(a.incompr ? K_PLAIN_INCOMPR : (libm ? K_PLAIN_LIBM : K_PLAIN_SCALAR));
-        int rc;
-        if (a.incompr) {
-            rc = libm ? dispatch_dim<R, true, true>(dim, gl, smem, st, a.pos, P, wtab, rec, nc,
-                                                    mps_c, !first, dst, sd, sp, split_stride, a.run_if)
-                      : dispatch_dim<R, true, false>(dim, gl, smem, st, a.pos, P, wtab, rec, nc,
-                                                     mps_c, !first, dst, sd, sp, split_stride, a.run_if);
-        } else {
-            rc = libm ? dispatch_dim<R, false, true>(dim, gl, smem, st, a.pos, P, wtab, rec, nc,
-                                                     mps_c, !first, dst, sd, sp, split_stride, a.run_if)
-                      : dispatch_dim<R, false, false>(dim, gl, smem, st, a.pos, P, wtab, rec, nc,
-                                                      mps_c, !first, dst, sd, sp, split_stride, a.run_if);
-        }
+        const int rc = dispatch_plain(shp.R, a.incompr, libm, dim,
+                                      dim3(static_cast<unsigned>(shp.bx), static_cast<unsigned>(s_used)),
+                                      st, l);
         tl.end();
         if (rc != GSC_OK) return rc;
-        first = 0;
         j0 += nc;
     } while (j0 < N);
 
@@ -635,67 +717,56 @@ int plain_run(DeviceCtx &ctx, const PlainArgs &a, cudaStream_t st) {
     return GSC_OK;
 }
 
-// ---- batched ensembles: tables and the persistent kernel ---------------------
-int batch_plain_tables(const BatchItem *items, const int64_t *mode_prefix, int64_t n_items,
-                       int64_t total_modes, void *wtab, double *rec, cudaStream_t st) {
+// ---- batched ensembles: records and the persistent kernel --------------------
+int batch_plain_tables(const BatchItem *items, int64_t n_items, int64_t total_modes, double *rec,
+                       cudaStream_t st) {
     if (total_modes == 0) return GSC_OK;
-    if (total_modes > 0x7fffffff) return set_error(GSC_ERR_INVALID, "too many modes in the batch");
     TimedLaunch tl(st);
     tl.begin(K_BATCH_TABLES);
-    batch_table_kernel<<<static_cast<unsigned>(total_modes), kM, 0, st>>>(
-        items, mode_prefix, n_items, static_cast<double2 *>(wtab), rec);
+    // enough warps for the items' mean group count, the larger items striding
+    const int64_t mean = (total_modes / kGroup + n_items) / n_items;
+    const unsigned gx = static_cast<unsigned>(std::min<int64_t>(64, std::max<int64_t>(1, mean / (kThreads / 32))));
+    batch_rec_kernel<<<dim3(gx, static_cast<unsigned>(std::min<int64_t>(n_items, 65535))), kThreads, 0, st>>>(
+        items, n_items, rec);
     tl.end();
     GSC_CUDA(cudaGetLastError());
     return GSC_OK;
 }
 
-size_t batch_plain_smem(int tile) { return 2 * static_cast<size_t>(tile) * (kM * 16 + kRec * 8); }
-
 namespace {
-using BatchPlainFn = void (*)(const BatchItem *, const BatchUnit *, int64_t, int *,
-                              const double2 *, const double *);
-BatchPlainFn batch_plain_fn(int R, int tile) {
-    if (tile == 8) {
-        if (R == 2) return batch_plain_kernel<2, 8>;
-        if (R == 4) return batch_plain_kernel<4, 8>;
-        if (R == 8) return batch_plain_kernel<8, 8>;
-    } else if (tile == 16) {
-        if (R == 2) return batch_plain_kernel<2, 16>;
-        if (R == 4) return batch_plain_kernel<4, 16>;
-    }
+using BatchPlainFn = void (*)(const BatchItem *, const BatchUnit *, int64_t, int *, const double *);
+BatchPlainFn batch_plain_fn(int R) {
+    if (R == 2) return batch_plain_kernel<2>;
+    if (R == 4) return batch_plain_kernel<4>;
+    if (R == 8) return batch_plain_kernel<8>;
     return nullptr;
-}
-int configure_batch_plain(BatchPlainFn fn, int tile) {
-    return smem_attr(reinterpret_cast<const void *>(fn), batch_plain_smem(tile));   // per device
 }
 }  // namespace
 
-bool batch_plain_config_ok(int R, int tile) { return batch_plain_fn(R, tile) != nullptr; }
+// The tile sizes that a caller may name (8 or 16 modes; 8 alone with 8 points
+// per thread); the kernels stage 32 modes whatever it is.
+bool batch_plain_config_ok(int R, int tile) {
+    return batch_plain_fn(R) != nullptr && (tile == 8 || (tile == 16 && R != 8));
+}
 
-int batch_plain_occupancy(int R, int tile, int device) {
-    BatchPlainFn fn = batch_plain_fn(R, tile);
+int batch_plain_occupancy(int R) {
+    BatchPlainFn fn = batch_plain_fn(R);
     if (!fn) return 0;
-    if (configure_batch_plain(fn, tile) != GSC_OK) return 0;
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kThreads, batch_plain_smem(tile)) !=
-        cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kThreads, 0) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
-    (void)device;
     return n;
 }
 
-int batch_plain_launch(int R, int tile, int blocks, const BatchItem *items,
-                       const BatchUnit *units, int64_t n_units, int *counter, const void *wtab,
-                       const double *rec, cudaStream_t st) {
-    BatchPlainFn fn = batch_plain_fn(R, tile);
+int batch_plain_launch(int R, int blocks, const BatchItem *items, const BatchUnit *units,
+                       int64_t n_units, int *counter, const double *rec, cudaStream_t st) {
+    BatchPlainFn fn = batch_plain_fn(R);
     if (!fn) return set_error(GSC_ERR_INVALID, "unsupported batch configuration");
-    GSC_TRY(configure_batch_plain(fn, tile));
     TimedLaunch tl(st);
     tl.begin(K_BATCH_PLAIN);
-    fn<<<blocks, kThreads, batch_plain_smem(tile), st>>>(items, units, n_units, counter,
-                                                         static_cast<const double2 *>(wtab), rec);
+    fn<<<blocks, kThreads, 0, st>>>(items, units, n_units, counter, rec);
     tl.end();
     GSC_CUDA(cudaGetLastError());
     return GSC_OK;
@@ -710,31 +781,20 @@ int batch_plain_launch(int R, int tile, int blocks, const BatchItem *items,
 // framework allocator already owns the whole device (a cudaMalloc from the
 // library would fail or fragment that pool), a real-time loop that cannot
 // afford to block in the driver's allocator, or a plug-in host that only
-// permits memory from its own arena.  For them the per-mode tables of the
+// permits memory from its own arena.  For them the mode records of the
 // plain kernel live in one fixed array compiled into the library, so a call
 // allocates nothing; the caller passes the inputs and the output as usual.
 //
-// The array (4 MiB of tables + 96 KiB of mode records, enough for 1024
-// modes) is held on every GPU that loads the library until the process
+// The array (144 KiB of mode records, enough for 1024 modes) is held on every GPU that loads the library until the process
 // exits.  All calls share it and it keeps the last call's contents; every
 // call rewrites the part it reads, so nothing has to start at zero.  Calls
 // whose kernels overlap on the GPU (different streams, no ordering between
 // them) race on the array.
 // ---------------------------------------------------------------------------
 static __device__ __align__(256) unsigned char
-    gsc_noalloc_scratch[gsc::kNoAllocModes *
-                        (gsc::kPlainTableBytesPerMode + gsc::kPlainRecBytesPerMode)];
+    gsc_noalloc_scratch[gsc::kNoAllocModes * gsc::kPlainRecBytesPerMode];
 
 namespace gsc {
-
-// the array is sliced below as kNoAllocModes tables of kM double2 followed by
-// kNoAllocModes records of kRec doubles: its size must follow those constants
-static_assert(kPlainTableBytesPerMode == kM * sizeof(double2) &&
-                  kPlainRecBytesPerMode == kRec * sizeof(double),
-              "the fixed table array is sized from the plain kernel's per-mode layout");
-static_assert(sizeof(gsc_noalloc_scratch) ==
-                  kNoAllocModes * (kM * sizeof(double2) + kRec * sizeof(double)),
-              "fixed table array size");
 
 static std::mutex g_noalloc_mu;
 static void *g_noalloc_addr[64] = {nullptr};
@@ -748,7 +808,7 @@ static int noalloc_address(int device, void **addr) {
     if (!g_noalloc_addr[device]) {
         void *p = nullptr;
         const cudaError_t e = cudaGetSymbolAddress(&p, gsc_noalloc_scratch);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(fixed table array)");
+        if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(fixed record array)");
         g_noalloc_addr[device] = p;
     }
     *addr = g_noalloc_addr[device];
@@ -761,26 +821,31 @@ int plain_noalloc_run(int device, const PlainArgs &a, cudaStream_t st) {
     if (N > kNoAllocModes)
         return set_error(GSC_ERR_INVALID, "gsc_summate_dev_noalloc takes at most " +
                                               std::to_string(kNoAllocModes) +
-                                              " modes per call (its fixed table array holds "
+                                              " modes per call (its fixed record array holds "
                                               "that many); split the modes over several calls "
                                               "or use gsc_summate_dev");
     if (P == 0) return GSC_OK;
     void *scratch = nullptr;
     GSC_TRY(noalloc_address(device, &scratch));
-    double2 *wtab = static_cast<double2 *>(scratch);
-    double *rec = reinterpret_cast<double *>(static_cast<unsigned char *>(scratch) +
-                                             kNoAllocModes * kM * sizeof(double2));
+    double *rec = static_cast<double *>(scratch);
     const int64_t bx = (P + kThreads * R - 1) / (kThreads * R);
     if (bx > 0x7fffffff) return set_error(GSC_ERR_INVALID, "too many points for one launch");
     if (N > 0) {
-        mode_table_kernel<<<static_cast<unsigned>(N), kM, 0, st>>>(a.cov, a.z1, a.z2, a.dim, N, 0,
-                                                                      0, 1, wtab, rec, nullptr);
+        plain_rec_kernel<<<static_cast<unsigned>((N + kThreads - 1) / kThreads), kThreads, 0, st>>>(
+            a.cov, a.z1, a.z2, static_cast<int>(a.dim), N, 0, N, 0, rec, nullptr);
         GSC_CUDA(cudaGetLastError());
     }
-    const size_t smem = 2 * (kTileModes * kM * 16 + kTileModes * kRec * 8);
     // one mode split: every point's modes are summed by one thread, in order
-    return dispatch_dim<R, false, false>(a.dim, dim3(static_cast<unsigned>(bx), 1), smem, st,
-                                         a.pos, P, wtab, rec, N, N, 0, a.out, P, a.out_sp, 0);
+    PlainLaunch l{};
+    l.pos = a.pos;
+    l.P = P;
+    l.rec = rec;
+    l.nc = N;
+    l.mps = N;
+    l.dst = a.out;
+    l.sd = P;
+    l.sp = a.out_sp;
+    return dispatch_plain(R, false, false, a.dim, dim3(static_cast<unsigned>(bx), 1), st, l);
 }
 
 }  // namespace gsc

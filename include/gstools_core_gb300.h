@@ -55,7 +55,8 @@ extern "C" {
 
 /* ---- computation forms ----------------------------------------------- */
 #define GSC_FORM_AUTO       0  /* library choice for the requested tolerance */
-#define GSC_FORM_PLAIN_F64  1  /* FP64 end to end, table-driven FP64 sincos   */
+#define GSC_FORM_PLAIN_F64  1  /* FP64 phases, cosines and sums of 32 modes in
+                                  64-bit fixed point, FP64 totals             */
 #define GSC_FORM_PLAIN_F64_LIBM 2  /* FP64 end to end on CUDA's sincos()    */
 #define GSC_FORM_SEP_F16X3  3  /* structured grids: separable contraction on
                                   tcgen05 tensor cores, both operands split
@@ -191,8 +192,8 @@ int gsc_summate_dev(const double *cov, const double *z1, const double *z2,
  * memory -- a host whose own allocator owns the whole GPU, a real-time loop
  * that cannot block in the driver's allocator, a plug-in host that hands out
  * memory only from its arena.  The call allocates nothing: the plain FP64
- * kernel's per-mode tables live in a fixed array inside the library
- * (4 MiB + 96 KiB, held on every GPU that loads the library until exit), so
+ * kernel's mode records live in a fixed array inside the library
+ * (144 KiB, held on every GPU that loads the library until exit), so
  * a call takes at most 1024 modes and returns GSC_ERR_INVALID beyond that.
  * Inputs and output are the caller's device arrays, as for gsc_summate_dev;
  * dim in {1, 2, 3}; forms AUTO or PLAIN_F64 only.  The first call on a
