@@ -45,7 +45,7 @@ const char *kernel_name(int32_t id) {
         "grid_expand", "sep_tc_f16x5", "mixed_modes", "mixed_scalar", "mixed_incompr",
         "mixed_f64phase", "sep_f64_dmma", "fourier_scale", "batch_tables", "batch_plain",
         "batch_mixed", "sample_modes", "sep_split", "copy_h2d", "copy_d2h", "interleave",
-        "mesh_check",
+        "mesh_check", "sep_f64_slices",
     };
     return (id >= 0 && id < K_COUNT) ? names[id] : "unknown";
 }

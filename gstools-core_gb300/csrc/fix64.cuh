@@ -163,4 +163,63 @@ __device__ __forceinline__ int64_t cos_fixed(uint64_t theta, const CosTable *tab
     return c - (p >> 6);
 }
 
+// cos and sin of 2 pi (theta - kFineOffset) / 2^64 in units of 2^-62, within
+// 1e-17: the same table with one more order of the cosine and 64-bit products,
+// for factor tables, where an error is shared by many sums.
+//   1 - cos(step rho) = f1 rho^2 (1 - f2 rho^2 + f3 rho^4)
+//   sin(step rho)     = step rho (1 - f4 rho^2 + f5 rho^4)
+// with the Taylor coefficients f1 = step^2 / 2, f2 = step^2 / 12, f3 =
+// step^4 / 360, f4 = step^2 / 6, f5 = step^4 / 120 (the sine's next term is
+// 8.4e-18).
+constexpr uint64_t kFineOffset = uint64_t(1) << 55;
+constexpr uint64_t kFine1 = 0x9de9e64df22ef2d2ull;     // f1 2^75
+constexpr uint64_t kFine2 = 0x34a34cc4a60fa646ull;     // f2 2^76
+constexpr uint64_t kFine3 = 0x000022a264558fb1ull;     // f3 2^75
+constexpr uint64_t kFine4 = 0x34a34cc4a60fa646ull;     // f4 2^75
+constexpr uint64_t kFine5 = 0x000033f396805789ull;     // f5 2^74
+__device__ __forceinline__ void cis_fine(uint64_t theta, const CosTable *tab, int64_t *cosine, int64_t *sine) {
+    const uint32_t a = static_cast<uint32_t>(theta >> 56);
+    const uint4 e = tab->wide[a], g = tab->wide[(a + 192) & 255];
+    const int64_t c = static_cast<int64_t>((static_cast<uint64_t>(e.y) << 32) | e.x);
+    const int64_t s = static_cast<int64_t>((static_cast<uint64_t>(g.y) << 32) | g.x);
+    // rho 2^64 and rho^2 2^65 (at most 2^63)
+    const int64_t rho = static_cast<int64_t>((theta << 8) ^ (uint64_t(1) << 63));
+    const uint64_t q = static_cast<uint64_t>(__mul64hi(rho, rho)) << 1;
+    // rho^2 (f2 - ..) in units of 2^-77, rho^2 (f4 - ..) of 2^-76
+    const uint64_t lv = __umul64hi(q, kFine2 - __umul64hi(q, kFine3));
+    const uint64_t ls = __umul64hi(q, kFine4 - __umul64hi(q, kFine5));
+    // rho^2 (1 - ..) of 2^-65 and the versine of 2^-76; rho (1 - ..) of 2^-64 and the sine of 2^-68
+    const uint64_t vq = q - (__umul64hi(q, lv) >> 13);
+    const int64_t ver = static_cast<int64_t>(__umul64hi(vq, kFine1));
+    const int64_t rs = rho - (__mul64hi(rho, static_cast<int64_t>(ls)) >> 12);
+    const int64_t sn = __mul64hi(rs, static_cast<int64_t>(kStep69 >> 1));
+    *cosine = c - (((__mul64hi(c, ver) >> 8) + __mul64hi(s, sn) + 8) >> 4);
+    *sine = s - (((__mul64hi(s, ver) >> 8) - __mul64hi(c, sn) + 8) >> 4);
+}
+
+// Finite z1, z2 as z1 + i z2 = amp 2^ez e^{i beta} (amp in [1/2, sqrt 2), or
+// 0): a first angle in FP32, its cosine and sine in 64 bits, then the remaining
+// rotation d (1e-7 rad) from the cross product.  An FP64 atan2 and hypot would
+// be a chain of several microseconds, and less exact.
+__device__ __forceinline__ void mode_angle(double z1, double z2, const CosTable *tab, double *amp,
+                                           int *ez, uint64_t *beta) {
+    *amp = 0.0;
+    *ez = 0;
+    *beta = 0;
+    const double zm = fmax(fabs(z1), fabs(z2));
+    if (zm == 0.0) return;
+    frexp(zm, ez);
+    const double y1 = ldexp(z1, -*ez), y2 = ldexp(z2, -*ez);
+    const float t = atan2f(static_cast<float>(y2), static_cast<float>(y1)) * 0.15915494f;   // turns
+    const uint64_t b = static_cast<uint64_t>(__float2ll_rn(t * 1099511627776.0f)) << 24;
+    const int64_t f1 = __double2ll_rn(y1 * 0x1p62), f2 = __double2ll_rn(y2 * 0x1p62);
+    int64_t c, s;
+    cis_fine(b + kFineOffset, tab, &c, &s);
+    const double along = static_cast<double>(__mul64hi(f1, c) + __mul64hi(f2, s));    // units 2^-60
+    const double across = static_cast<double>(__mul64hi(f2, c) - __mul64hi(f1, s));
+    const double d = across / along;
+    *amp = fma(along, 0.5 * d * d, along) * 0x1p-60;
+    *beta = b + static_cast<uint64_t>(__double2ll_rn(d * 2.935890503282001e18));      // 2^64 / 2 pi
+}
+
 }  // namespace gsc

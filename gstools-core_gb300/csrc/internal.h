@@ -63,6 +63,7 @@ enum KernelId : int32_t {
     K_COPY_D2H = 23,       // device-to-host copies of a host-pointer call (not a kernel)
     K_INTERLEAVE = 24,     // (nout, P) rows to the (P, nout) layout of a Fortran-ordered result
     K_MESH_CHECK = 25,     // the device's share of the check of a flattened mesh
+    K_SEP_F64_SLICES = 26, // separable contraction in 9-bit slices on tcgen05 (sep_f64)
     K_COUNT
 };
 const char *kernel_name(int32_t id);
@@ -276,7 +277,15 @@ struct SepArgs {
     const std::function<int(int64_t lo, int64_t hi)> *on_rows = nullptr;
 };
 int sep_tc_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st);
-int sep_f64_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st);   // separable_f64.cu
+// GSC_FORM_SEP_F64: the slices (separable_slices.cu), with the FP64 MMA
+// (separable_f64.cu) queued behind for inputs outside their range; the FP64 MMA
+// alone for a call predicated on run_if
+int sep_f64_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st);
+int sep_slices_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st);
+// The FP64 MMA's scratch bytes, and its launches on scratch `base`, which do
+// nothing while *run_if is 0 (run_if null: always run)
+size_t sep_f64_scratch(const SepArgs &a);
+int sep_f64_launch(const SepArgs &a, unsigned char *base, const int *run_if, cudaStream_t st);
 
 // ---- batched ensembles (batch.cu, with kernels in plain.cu / mixed.cu) ------
 // One realization of an ensemble as the device kernels see it.

@@ -70,9 +70,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 // ---------------------------------------------------------------------------
 // Mode records.  One warp per group of 32 modes, lane = mode (live: it exists);
-// all lanes call.  Everything but the last few FP64 operations is integer
-// arithmetic: an FP64 atan2 and hypot would be a chain of several microseconds
-// and less exact.
+// all lanes call.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void rec_group(const double *__restrict__ cov, int64_t n_modes, int dim,
                                           int64_t j, bool live, double z1, double z2, int incompr,
@@ -91,26 +89,10 @@ __device__ __forceinline__ void rec_group(const double *__restrict__ cov, int64_
         w[2] = -__dmul_rn(k[2], k_2);
         regular = regular && isfinite(w[0]) && isfinite(w[1]) && isfinite(w[2]);
     }
-    // z1 + i z2 = A e^{i beta}: a first angle in FP32, its cosine and sine in
-    // 64 bits, then the remaining rotation d (1e-7 rad) from the cross product
     uint64_t beta = 0;
     double amp = 0.0;                                            // A 2^-ez
     int ez = 0;
-    const double zm = fmax(fabs(z1), fabs(z2));
-    if (regular && zm > 0.0) {
-        frexp(zm, &ez);
-        const double y1 = ldexp(z1, -ez), y2 = ldexp(z2, -ez);
-        const float t = atan2f(static_cast<float>(y2), static_cast<float>(y1)) * 0.15915494f;   // turns
-        beta = static_cast<uint64_t>(__float2ll_rn(t * 1099511627776.0f)) << 24;
-        const int64_t f1 = __double2ll_rn(y1 * 0x1p62), f2 = __double2ll_rn(y2 * 0x1p62);
-        const int64_t c = cos_fixed(beta + kCosOffset, tab);
-        const int64_t s = cos_fixed(beta - (uint64_t(1) << 62) + kCosOffset, tab);
-        const double along = static_cast<double>(__mul64hi(f1, c) + __mul64hi(f2, s));    // units 2^-60
-        const double across = static_cast<double>(__mul64hi(f2, c) - __mul64hi(f1, s));
-        const double d = across / along;
-        amp = fma(along, 0.5 * d * d, along) * 0x1p-60;
-        beta += static_cast<uint64_t>(__double2ll_rn(d * 2.935890503282001e18));          // 2^64 / 2 pi
-    }
+    if (regular) mode_angle(z1, z2, tab, &amp, &ez, &beta);
     const int nout = incompr ? dim : 1;
     double a[3] = {incompr ? amp * w[0] : amp, amp * w[1], amp * w[2]};
     double scale[3] = {0.0, 0.0, 0.0};
@@ -632,7 +614,6 @@ int interleave_rows(const double *src, int64_t nout, int64_t P, int64_t p0, int6
 }
 
 int plain_run(DeviceCtx &ctx, const PlainArgs &a, cudaStream_t st) {
-    constexpr int R = 4;
     const int64_t P = a.n_points, N = a.n_modes, dim = a.dim;
     if (P == 0) return GSC_OK;
     const int64_t nout = a.incompr ? dim : 1;

@@ -5,8 +5,13 @@
 // K = 2N: rows F[b, (2j, 2j+1)] = (Re, Im)(s_a[j] B[b, j]), columns
 // G[c, (2j, 2j+1)] = (Re, -Im)(p_c C[c, j])), but every operand, product and
 // sum is FP64, so the result agrees with the reference's summator
-// (src/field.rs:37-65, :97-182 on the expanded grid) to FP64 round-off while
-// doing 2 * points * 2N FLOPs instead of a sincos per point*mode.
+// (src/field.rs:37-65, :97-182 on the expanded grid) to FP64 round-off, for
+// any inputs.  At 1.1 TFLOP/s it is the way out for what the sliced form
+// (separable_slices.cu) does not take (values that are not finite, phases of
+// 2^32 and more, calls without modes) and for grids that the x5 form flagged:
+// both launches of a call are queued behind the fast form's and leave at once
+// unless the word at run_if is set.  They run a fixed number of blocks over all
+// tiles, so that leaving costs the launches alone.
 //
 // Tiles: one CTA per 64 x 64 output tile of one X_a, 4 warps of 32 x 32,
 // K staged 32 at a time through shared memory (rows padded to 33 doubles to
@@ -26,6 +31,7 @@ namespace {
 constexpr int TM = 64, TN = 64, TK = 32;     // tile rows, columns, K per stage
 constexpr int LDS = TK + 1;                  // padded shared-memory row (doubles)
 constexpr int kF64Threads = 128;
+constexpr int kF64Grid = 152 * 4;            // blocks that fit at once
 
 struct F64Tab {
     const double *cov, *z1, *z2;
@@ -40,10 +46,7 @@ struct F64Tab {
     const int *run_if; // null, or a device word: the launch does nothing while it is 0
 };
 
-__global__ void f64_svec_kernel(F64Tab t) {
-    if (t.run_if && *t.run_if == 0) return;
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= static_cast<int64_t>(t.nb) * t.n_modes) return;
+__device__ void f64_svec_entry(const F64Tab &t, int64_t i) {
     const int b = static_cast<int>(i / t.n_modes), j = static_cast<int>(i % t.n_modes);
     double re = t.z1[j], im = -t.z2[j];
     if (t.dim == 3) {
@@ -56,21 +59,15 @@ __global__ void f64_svec_kernel(F64Tab t) {
     t.svec[i] = make_double2(re, im);
 }
 
-__global__ void f64_btab_kernel(F64Tab t) {
-    if (t.run_if && *t.run_if == 0) return;
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= static_cast<int64_t>(t.n_modes) * t.nm) return;
+__device__ void f64_btab_entry(const F64Tab &t, int64_t i) {
     const int j = static_cast<int>(i / t.nm), m = static_cast<int>(i % t.nm);
     double s, c;
     sincos(t.cov[t.km_dim * t.n_modes + j] * t.ax_m[m], &s, &c);
     t.btab[i] = make_double2(c, s);
 }
 
-__global__ void f64_gtab_kernel(F64Tab t) {
-    if (t.run_if && *t.run_if == 0) return;
+__device__ void f64_gtab_entry(const F64Tab &t, int64_t i) {
     const int half_k = t.k_pad / 2;
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= static_cast<int64_t>(t.ncn_pad) * half_k) return;
     const int row = static_cast<int>(i / half_k), j = static_cast<int>(i % half_k);
     double re = 0.0, im = 0.0;
     if (row < t.ncomp * t.nn && j < t.n_modes) {
@@ -96,6 +93,19 @@ __global__ void f64_gtab_kernel(F64Tab t) {
     t.g[static_cast<int64_t>(row) * t.k_pad + 2 * j + 1] = im;
 }
 
+// s, B and G tables: a fixed grid strides over all entries
+__global__ void __launch_bounds__(256) f64_tables_kernel(F64Tab t) {
+    if (t.run_if && *t.run_if == 0) return;
+    const int64_t n1 = static_cast<int64_t>(t.nb) * t.n_modes, n2 = static_cast<int64_t>(t.n_modes) * t.nm;
+    const int64_t n3 = static_cast<int64_t>(t.ncn_pad) * (t.k_pad / 2);
+    const int64_t step = static_cast<int64_t>(gridDim.x) * 256;
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; i < n1 + n2 + n3; i += step) {
+        if (i < n1) f64_svec_entry(t, i);
+        else if (i < n1 + n2) f64_btab_entry(t, i - n1);
+        else f64_gtab_entry(t, i - n1 - n2);
+    }
+}
+
 __device__ __forceinline__ void dmma_8x8x4(double &d0, double &d1, double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                  : "+d"(d0), "+d"(d1)
@@ -107,6 +117,7 @@ struct F64Params {
     const double *g;
     int n_modes, nm, nn, ncn, k_pad;
     int m_tiles, n_tiles;
+    int64_t tiles;       // nb * m_tiles * n_tiles
     double *out;
     int64_t comp_stride, batch_stride, row_stride;
     const int *run_if;   // as in F64Tab
@@ -118,73 +129,74 @@ sep_f64_kernel(const F64Params p) {
     __shared__ double As[TM * LDS];
     __shared__ double Bs[TN * LDS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int tile = blockIdx.x;
-    const int nt = tile % p.n_tiles;
-    tile /= p.n_tiles;
-    const int mt = tile % p.m_tiles;
-    const int b = tile / p.m_tiles;
-    const int m0 = mt * TM, n0 = nt * TN;
     const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;   // warp's 32 x 32 sub-tile
     const int grp = lane >> 2, tig = lane & 3;
 
-    double acc[4][4][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int64_t tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
+        const int nt = static_cast<int>(tile % p.n_tiles);
+        const int64_t tm = tile / p.n_tiles;
+        const int mt = static_cast<int>(tm % p.m_tiles), b = static_cast<int>(tm / p.m_tiles);
+        const int m0 = mt * TM, n0 = nt * TN;
 
-    const double2 *sv = p.svec + static_cast<int64_t>(b) * p.n_modes;
-    for (int k0 = 0; k0 < p.k_pad; k0 += TK) {
-        __syncthreads();
-        // F tile: 64 rows x 16 modes, (Re, Im) interleaved along K
-        for (int e = tid; e < TM * (TK / 2); e += kF64Threads) {
-            const int r = e % TM, jl = e / TM;
-            const int j = k0 / 2 + jl, m = m0 + r;
-            double re = 0.0, im = 0.0;
-            if (m < p.nm && j < p.n_modes) {
-                const double2 bt = p.btab[static_cast<int64_t>(j) * p.nm + m];
-                const double2 s = sv[j];
-                re = bt.x * s.x - bt.y * s.y;
-                im = bt.x * s.y + bt.y * s.x;
-            }
-            As[r * LDS + 2 * jl] = re;
-            As[r * LDS + 2 * jl + 1] = im;
-        }
-        // G tile: 64 rows x 32 K
-        for (int e = tid; e < TN * TK; e += kF64Threads) {
-            const int r = e / TK, k = e % TK;
-            Bs[r * LDS + k] = p.g[static_cast<int64_t>(n0 + r) * p.k_pad + k0 + k];
-        }
-        __syncthreads();
+        double acc[4][4][2];
 #pragma unroll
-        for (int kk = 0; kk < TK; kk += 4) {
-            double a[4], bb[4];
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[(wm + 8 * i + grp) * LDS + kk + tig];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) bb[j] = Bs[(wn + 8 * j + grp) * LDS + kk + tig];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], bb[j]);
-        }
-    }
+            for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
-    double *ob = p.out + static_cast<int64_t>(b) * p.batch_stride;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + wm + 8 * i + grp;
-        if (m >= p.nm) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int gn = n0 + wn + 8 * j + 2 * tig + h;
-                if (gn >= p.ncn) continue;
-                const int comp = gn / p.nn;
-                ob[static_cast<int64_t>(m) * p.row_stride + comp * p.comp_stride + (gn - comp * p.nn)] =
-                    acc[i][j][h];
+        const double2 *sv = p.svec + static_cast<int64_t>(b) * p.n_modes;
+        for (int k0 = 0; k0 < p.k_pad; k0 += TK) {
+            __syncthreads();
+            // F tile: 64 rows x 16 modes, (Re, Im) interleaved along K
+            for (int e = tid; e < TM * (TK / 2); e += kF64Threads) {
+                const int r = e % TM, jl = e / TM;
+                const int j = k0 / 2 + jl, m = m0 + r;
+                double re = 0.0, im = 0.0;
+                if (m < p.nm && j < p.n_modes) {
+                    const double2 bt = p.btab[static_cast<int64_t>(j) * p.nm + m];
+                    const double2 s = sv[j];
+                    re = bt.x * s.x - bt.y * s.y;
+                    im = bt.x * s.y + bt.y * s.x;
+                }
+                As[r * LDS + 2 * jl] = re;
+                As[r * LDS + 2 * jl + 1] = im;
             }
+            // G tile: 64 rows x 32 K
+            for (int e = tid; e < TN * TK; e += kF64Threads) {
+                const int r = e / TK, k = e % TK;
+                Bs[r * LDS + k] = p.g[static_cast<int64_t>(n0 + r) * p.k_pad + k0 + k];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int kk = 0; kk < TK; kk += 4) {
+                double a[4], bb[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = As[(wm + 8 * i + grp) * LDS + kk + tig];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) bb[j] = Bs[(wn + 8 * j + grp) * LDS + kk + tig];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], bb[j]);
+            }
+        }
+
+        double *ob = p.out + static_cast<int64_t>(b) * p.batch_stride;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int m = m0 + wm + 8 * i + grp;
+            if (m >= p.nm) continue;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int gn = n0 + wn + 8 * j + 2 * tig + h;
+                    if (gn >= p.ncn) continue;
+                    const int comp = gn / p.nn;
+                    ob[static_cast<int64_t>(m) * p.row_stride + comp * p.comp_stride + (gn - comp * p.nn)] =
+                        acc[i][j][h];
+                }
+        }
     }
 }
 
@@ -192,85 +204,98 @@ size_t up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 }  // namespace
 
-int sep_f64_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
-    const int dim = static_cast<int>(a.dim);
-    const int N = static_cast<int>(a.n_modes);
-    const int ncomp = a.incompr ? dim : 1;
-    const int nb = dim == 3 ? static_cast<int>(a.n[0]) : 1;
-    const int nm = static_cast<int>(dim == 3 ? a.n[1] : a.n[0]);
-    const int nn = static_cast<int>(dim == 3 ? a.n[2] : a.n[1]);
-    const int64_t P = static_cast<int64_t>(nb) * nm * nn;
-    if (P == 0) return GSC_OK;
-    const int k_pad = std::max(TK, (2 * N + TK - 1) / TK * TK);
-    const int ncn = ncomp * nn;
-    const int n_tiles = (ncn + TN - 1) / TN, m_tiles = (nm + TM - 1) / TM;
-    const int ncn_pad = n_tiles * TN;
+namespace {
+struct F64Shape {
+    int dim, N, ncomp, nb, nm, nn, k_pad, ncn, n_tiles, m_tiles, ncn_pad;
+    int64_t P;
+    size_t off_btab, off_g, total;     // s at 0
+};
+F64Shape f64_shape(const SepArgs &a) {
+    F64Shape s;
+    s.dim = static_cast<int>(a.dim);
+    s.N = static_cast<int>(a.n_modes);
+    s.ncomp = a.incompr ? s.dim : 1;
+    s.nb = s.dim == 3 ? static_cast<int>(a.n[0]) : 1;
+    s.nm = static_cast<int>(s.dim == 3 ? a.n[1] : a.n[0]);
+    s.nn = static_cast<int>(s.dim == 3 ? a.n[2] : a.n[1]);
+    s.P = static_cast<int64_t>(s.nb) * s.nm * s.nn;
+    s.k_pad = std::max(TK, (2 * s.N + TK - 1) / TK * TK);
+    s.ncn = s.ncomp * s.nn;
+    s.n_tiles = (s.ncn + TN - 1) / TN;
+    s.m_tiles = (s.nm + TM - 1) / TM;
+    s.ncn_pad = s.n_tiles * TN;
+    s.off_btab = up(sizeof(double2) * s.nb * static_cast<size_t>(s.N), 256);
+    s.off_g = up(s.off_btab + sizeof(double2) * static_cast<size_t>(s.N) * s.nm, 256);
+    s.total = s.off_g + sizeof(double) * static_cast<size_t>(s.ncn_pad) * s.k_pad;
+    return s;
+}
+}  // namespace
 
-    const size_t off_svec = 0;
-    const size_t off_btab = up(off_svec + sizeof(double2) * nb * static_cast<size_t>(N), 256);
-    const size_t off_g = up(off_btab + sizeof(double2) * static_cast<size_t>(N) * nm, 256);
-    const size_t total = off_g + sizeof(double) * static_cast<size_t>(ncn_pad) * k_pad;
-    GSC_TRY(ensure_dev(ctx, ctx.scratch, total));
-    GSC_CUDA(cudaStreamWaitEvent(st, ctx.scratch_ready, 0));
-    unsigned char *base = static_cast<unsigned char *>(ctx.scratch.ptr);
+size_t sep_f64_scratch(const SepArgs &a) { return f64_shape(a).total; }
 
+int sep_f64_launch(const SepArgs &a, unsigned char *base, const int *run_if, cudaStream_t st) {
+    const F64Shape s = f64_shape(a);
     F64Tab t;
     t.cov = a.cov;
     t.z1 = a.z1;
     t.z2 = a.z2;
-    t.dim = dim;
-    t.n_modes = N;
-    t.ax_b = dim == 3 ? a.axis[0] : nullptr;
-    t.ax_m = dim == 3 ? a.axis[1] : a.axis[0];
-    t.ax_n = dim == 3 ? a.axis[2] : a.axis[1];
+    t.dim = s.dim;
+    t.n_modes = s.N;
+    t.ax_b = s.dim == 3 ? a.axis[0] : nullptr;
+    t.ax_m = s.dim == 3 ? a.axis[1] : a.axis[0];
+    t.ax_n = s.dim == 3 ? a.axis[2] : a.axis[1];
     t.kb_dim = 0;
-    t.km_dim = dim == 3 ? 1 : 0;
-    t.kn_dim = dim == 3 ? 2 : 1;
-    t.nb = nb;
-    t.nm = nm;
-    t.nn = nn;
-    t.ncomp = ncomp;
+    t.km_dim = s.dim == 3 ? 1 : 0;
+    t.kn_dim = s.dim == 3 ? 2 : 1;
+    t.nb = s.nb;
+    t.nm = s.nm;
+    t.nn = s.nn;
+    t.ncomp = s.ncomp;
     t.incompr = a.incompr ? 1 : 0;
-    t.k_pad = k_pad;
-    t.ncn_pad = ncn_pad;
-    t.svec = reinterpret_cast<double2 *>(base + off_svec);
-    t.btab = reinterpret_cast<double2 *>(base + off_btab);
-    t.g = reinterpret_cast<double *>(base + off_g);
-    t.run_if = a.run_if;
-    {
-        TimedLaunch tl(st);
-        tl.begin(K_SEP_TABLES);
-        const int64_t n1 = static_cast<int64_t>(nb) * N, n2 = static_cast<int64_t>(N) * nm;
-        const int64_t n3 = static_cast<int64_t>(ncn_pad) * (k_pad / 2);
-        if (n1 > 0) f64_svec_kernel<<<static_cast<unsigned>((n1 + 255) / 256), 256, 0, st>>>(t);
-        if (n2 > 0) f64_btab_kernel<<<static_cast<unsigned>((n2 + 255) / 256), 256, 0, st>>>(t);
-        f64_gtab_kernel<<<static_cast<unsigned>((n3 + 255) / 256), 256, 0, st>>>(t);
-        tl.end();
-        GSC_CUDA(cudaGetLastError());
-    }
+    t.k_pad = s.k_pad;
+    t.ncn_pad = s.ncn_pad;
+    t.svec = reinterpret_cast<double2 *>(base);
+    t.btab = reinterpret_cast<double2 *>(base + s.off_btab);
+    t.g = reinterpret_cast<double *>(base + s.off_g);
+    t.run_if = run_if;
     F64Params p;
     p.svec = t.svec;
     p.btab = t.btab;
     p.g = t.g;
-    p.n_modes = N;
-    p.nm = nm;
-    p.nn = nn;
-    p.ncn = ncn;
-    p.k_pad = k_pad;
-    p.m_tiles = m_tiles;
-    p.n_tiles = n_tiles;
+    p.n_modes = s.N;
+    p.nm = s.nm;
+    p.nn = s.nn;
+    p.ncn = s.ncn;
+    p.k_pad = s.k_pad;
+    p.m_tiles = s.m_tiles;
+    p.n_tiles = s.n_tiles;
+    p.tiles = static_cast<int64_t>(s.nb) * s.m_tiles * s.n_tiles;
     p.out = a.out;
-    p.comp_stride = P;
-    p.batch_stride = static_cast<int64_t>(nm) * nn;
-    p.row_stride = nn;
-    p.run_if = a.run_if;
-    const int64_t grid = static_cast<int64_t>(nb) * m_tiles * n_tiles;
-    if (grid > 0x7fffffff) return set_error(GSC_ERR_INVALID, "grid too large");
+    p.comp_stride = s.P;
+    p.batch_stride = static_cast<int64_t>(s.nm) * s.nn;
+    p.row_stride = s.nn;
+    p.run_if = run_if;
+    {
+        TimedLaunch tl(st);
+        tl.begin(K_SEP_TABLES);
+        f64_tables_kernel<<<kF64Grid, 256, 0, st>>>(t);
+        tl.end();
+        GSC_CUDA(cudaGetLastError());
+    }
     TimedLaunch tl(st);
     tl.begin(K_SEP_F64);
-    sep_f64_kernel<<<static_cast<unsigned>(grid), kF64Threads, 0, st>>>(p);
+    sep_f64_kernel<<<static_cast<unsigned>(std::min<int64_t>(p.tiles, kF64Grid)), kF64Threads, 0, st>>>(p);
     tl.end();
     GSC_CUDA(cudaGetLastError());
+    return GSC_OK;
+}
+
+int sep_f64_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
+    if (a.n[0] * a.n[1] * (a.dim == 3 ? a.n[2] : 1) == 0) return GSC_OK;
+    if (!a.run_if && a.n_modes > 0) return sep_slices_run(ctx, a, st);
+    GSC_TRY(ensure_dev(ctx, ctx.scratch, sep_f64_scratch(a)));
+    GSC_CUDA(cudaStreamWaitEvent(st, ctx.scratch_ready, 0));
+    GSC_TRY(sep_f64_launch(a, static_cast<unsigned char *>(ctx.scratch.ptr), a.run_if, st));
     GSC_CUDA(cudaEventRecord(ctx.scratch_ready, st));
     return GSC_OK;
 }

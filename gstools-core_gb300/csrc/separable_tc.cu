@@ -375,7 +375,7 @@ sep_tc_kernel(const __grid_constant__ CUtensorMap map_ghi,
         }
     } else if (warp == kMmaWarp) {
         // ---- MMA issue -------------------------------------------------------
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = idesc_f16(BM, BN, BF16);
             bool ok = true;
             for (int kb = 0; kb < KB; ++kb) {
@@ -1127,7 +1127,7 @@ sep_x5_kernel(const __grid_constant__ CUtensorMap out_map, const X5Params xp) {
                 for (int i = issued_b > X5_STAGES ? issued_b - X5_STAGES : 0; i < issued_b; ++i)
                     mbar_wait_drain(&b_full[i % X5_STAGES], (i / X5_STAGES) & 1, p.status);
             }
-        } else if (warp == kMmaWarpX5 && lane == 0) {
+        } else if (warp == kMmaWarpX5 && elect_one()) {
             // ---- MMA ---------------------------------------------------------
             const uint32_t idesc = idesc_f16(BM, BNX, false);
             bool ok = true;

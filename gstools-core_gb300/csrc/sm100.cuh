@@ -108,6 +108,17 @@ __device__ __forceinline__ bool mbar_wait_drain(uint64_t *bar, uint32_t parity, 
     return true;
 }
 
+// One lane of a converged warp.  Code that only this lane runs is known to the
+// compiler to have one thread, so tcgen05 operands stay in uniform registers;
+// under `lane == 0` every MMA moved its descriptors there first, and an MMA
+// took at least 47 clocks to issue (87 with the descriptors computed around
+// it), more than the 40 to 128 that 128 x 80..256 x 16 needs.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
+
 // ---- proxies -------------------------------------------------------------------
 // Generic-proxy shared-memory writes made visible to the async proxy (MMA).
 __device__ __forceinline__ void fence_proxy_async_smem() {
@@ -192,6 +203,28 @@ __device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uin
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+// The same with the A operand kept in the collector buffer (fill) and read from
+// it again by the next MMAs (reuse) instead of from shared memory: A must be the
+// same matrix.  An MMA of 128 x N x 16 takes N / 2 clocks, or what 128 bytes per
+// clock make of its operands: (4096 + 32 N) / 128 without reuse, 32 N / 128 with.
+template <bool REUSE>
+__device__ __forceinline__ void mma_f16_ss_keep(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                                uint32_t idesc, uint32_t accumulate) {
+    if constexpr (REUSE)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16.collector::a::use [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+            "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16.collector::a::fill [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+            "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
 }
 // Arrives once on `bar` when all previously issued tcgen05.mma of this thread complete.
 __device__ __forceinline__ void mma_commit(uint64_t *bar) {

@@ -84,9 +84,12 @@ extern "C" {
                                   turns is flagged (see gsc_device_status)  */
 #define GSC_FORM_MIXED_F64PHASE 7 /* as GSC_FORM_MIXED with the phase and its
                                   reduction in FP64                          */
-#define GSC_FORM_SEP_F64    8  /* structured grids: separable contraction in
-                                  FP64 on the double-precision MMA; FP64
-                                  round-off (below 1e-12 of the field RMS)   */
+#define GSC_FORM_SEP_F64    8  /* structured grids: separable contraction to
+                                  FP64 round-off (below 1e-12 of the field
+                                  RMS), as 9-bit slices summed exactly on
+                                  tcgen05 tensor cores; the double-precision
+                                  MMA for values that are not finite and
+                                  phases of 2^32 and more                    */
 
 /* ---- flags ----------------------------------------------------------- */
 #define GSC_FLAG_TIMING     1  /* record per-kernel CUDA-event timings      */
