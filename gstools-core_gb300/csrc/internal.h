@@ -322,7 +322,7 @@ int batch_plain_launch(int R, int blocks, const BatchItem *items, const BatchUni
 int batch_mixed_launch(int R, bool f64phase, int blocks, const BatchItem *items,
                        const BatchUnit *units, int64_t n_units, int *counter, const float *rec,
                        const double *rec64, cudaStream_t st);
-constexpr int64_t kPlainRecBytesPerMode = 18 * 8;
+constexpr int64_t kPlainRecBytesPerMode = 20 * 8;
 constexpr int kPlainGroupModes = 32;   // modes summed as integers of one scale: ranges start on a multiple
 constexpr int64_t kMixedRecBytesPerMode = 20 * 4;
 constexpr int64_t kMixedRec64BytesPerMode = 4 * 8;

@@ -9,17 +9,23 @@
 //
 // Design.  GB300's FP64 pipe issues 2 lanes per clock and SM, so only what
 // needs its rounding stays on it; the rest runs on the integer pipes beside it:
-//  * phase k.x in FP64, formed exactly as the reference forms it:
-//    ((k0*x0 + k1*x1) + k2*x2), no FMA, so every phase has the reference's
-//    bits (src/field.rs:57, src/short_vec.rs:30-33): 2d - 1 instructions;
+//  * phase k.x with the reference's bits: ((k0*x0 + k1*x1) + k2*x2), no FMA
+//    (src/field.rs:57, src/short_vec.rs:30-33).  The first product and the sums
+//    are FP64 instructions; the other products are formed and rounded by
+//    integer instructions (rn_product), which overlap them;
 //  * z1 cos + z2 sin = A cos(phase - beta), A = |z1 + i z2| and beta its
 //    angle, set up per mode (plain_rec_kernel); the phase becomes a 64-bit
 //    fraction of a turn and its cosine a 64-bit integer (fix64.cuh: 1.2e-16
 //    RMS), one integer multiply by A (scaled by the largest A of 32 modes, to
 //    2^-57 of it) and a 64-bit sum over those 32 modes, which is exact; one
 //    FP64 multiply-add per 32 modes adds it to the point's total.
-//    The FP64 polynomials, table products and sums that this replaces were 18
-//    FP64 instructions per point*mode for d = 3 (16 for d = 2); @@FIG@@
+//    An FP64 evaluation (phase, table look-up, polynomials, sum) is 18 FP64
+//    instructions per point*mode for d = 3 and 16 for d = 2; this one has 3 and
+//    2.  Integer issue bounds the kernel now (a mode's 110 to 190 integer
+//    instructions against 77 clocks for each FP64 one): 100,000 2-D points x
+//    1000 modes 3391 -> 620 us, 250,007 3-D points x 1999 modes 18.86 -> 3.54 ms
+//    (4.89 with all products on the FP64 pipe), and the error against 64-bit
+//    sums fell from 1.7e-15 to 7e-16;
 //  * phases of 2^32 and more, and modes with a NaN or an infinity, take CUDA's
 //    sincos() and FP64 sums for that mode (the same test for a whole warp);
 //  * mode records (96 bytes) are staged 32 at a time into shared memory with
@@ -48,15 +54,17 @@ static_assert(kThreads == kBatchThreads, "batch units assume the plain block siz
 static_assert(kGroup == 32, "a warp builds the records of a group");
 
 // Mode record (8-byte words): what the sums read from shared memory, then the
-// FP64 weights of the exact path.
-//   k0 k1 | k2, |k| bound (FP32) | -beta + kCosOffset, A0 | A1 A2 | s0 s1 | s2 -
-//   z1 z2 | w0 w1 | w2 -
-// A_i = A w_i (A alone for the scalar field) as an integer of units s_i 2^-8
-// held in two words {high, low / 2}; s_i = 2^(e_i - 56), 2^(e_i) above every
-// |A_i| of the mode's group of 32.  The bound is infinite for a mode of the
-// exact path.
-constexpr int kRec = 18, kRecStaged = 12;
-enum { R_K0 = 0, R_K2 = 2, R_KABS = 3, R_BETA = 4, R_A0 = 5, R_S0 = 8, R_Z1 = 12, R_Z2 = 13, R_W0 = 14 };
+// FP64 values of the exact path.
+//   k0, k1 mantissa | k2 mantissa, k1 and k2 exponents | kCosOffset - beta, A0 |
+//   A1 A2 | s0 s1 | s2, |k| bound (FP32)
+//   z1 z2 | w0 w1 | w2 k1 | k2 -
+// k1 and k2 as factors of rn_product (mantissas {high, low}).  A_i = A w_i (A
+// alone for the scalar field) as an integer of units s_i 2^-8 held in two words
+// {high, low / 2}; s_i = 2^(e_i - 56), 2^(e_i) above every |A_i| of the mode's
+// group of 32.  The bound is infinite for a mode of the exact path.
+constexpr int kRec = 20, kRecStaged = 12;
+enum { R_K0 = 0, R_M1 = 1, R_M2 = 2, R_EXP = 3, R_BETA = 4, R_A0 = 5, R_S0 = 8, R_KABS = 11,
+       R_Z1 = 12, R_Z2 = 13, R_W0 = 14, R_K1 = 17, R_K2 = 18 };
 static_assert(kRec * 8 == kPlainRecBytesPerMode, "record layout");
 constexpr float kFastPhase = 4.29e9f;               // |k| |x| bound of the integer path, below 2^32
 
@@ -78,7 +86,7 @@ __device__ __forceinline__ void rec_group(const double *__restrict__ cov, int64_
     double k[3] = {0.0, 0.0, 0.0}, w[3] = {0.0, 0.0, 0.0};
     if (live)
         for (int d = 0; d < dim && d < 3; ++d) k[d] = cov[d * n_modes + j];
-    bool regular = isfinite(z1) && isfinite(z2) && isfinite(k[0]) && isfinite(k[1]) && isfinite(k[2]);
+    bool regular = isfinite(z1) && isfinite(z2) && isfinite(k[0]) && factor_in_range(k[1]) && factor_in_range(k[2]);
     if (incompr) {
         // src/field.rs:138: k_2 = k0 / k.k, ShortVec::dot order, no FMA
         double kk = 0.0;
@@ -115,9 +123,11 @@ __device__ __forceinline__ void rec_group(const double *__restrict__ cov, int64_
         scale[i] = ldexp(1.0, eg - 56);
     }
     if (!live) return;
+    const Factor f1 = factor_of(k[1]), f2 = factor_of(k[2]);
     r[R_K0] = k[0];
-    r[R_K0 + 1] = k[1];
-    r[R_K2] = k[2];
+    r[R_M1] = __hiloint2double(static_cast<int>(f1.m0), static_cast<int>(f1.m1));
+    r[R_M2] = __hiloint2double(static_cast<int>(f2.m0), static_cast<int>(f2.m1));
+    r[R_EXP] = __hiloint2double(static_cast<int>(f2.e), static_cast<int>(f1.e));
     const float kabs = regular ? __double2float_ru(fabs(k[0]) + fabs(k[1]) + fabs(k[2]))
                                : __int_as_float(0x7f800000);
     r[R_KABS] = __hiloint2double(0, __float_as_int(kabs));
@@ -129,10 +139,11 @@ __device__ __forceinline__ void rec_group(const double *__restrict__ cov, int64_
         r[R_S0 + i] = scale[i];
         r[R_W0 + i] = w[i];
     }
-    r[R_S0 + 3] = 0.0;
     r[R_Z1] = z1;
     r[R_Z2] = z2;
-    r[R_W0 + 3] = 0.0;
+    r[R_K1] = k[1];
+    r[R_K2] = k[2];
+    r[kRec - 1] = 0.0;
 }
 
 // Records of modes [j0, j0 + nc); grid ceil(nc / kThreads), j0 a multiple of 32.
@@ -219,7 +230,10 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
     };
     if (jb < je) stage_tile(0, jb);
 
-    double x[R][D];
+    // x0 as FP64, the other coordinates as factors of integer products (LIBM:
+    // read from pos where they are needed)
+    double x0[R];
+    Factor xf[R][D > 1 ? D - 1 : 1];
     double acc[R][NOUT];
     double xabs = 0.0;
     bool bad[R];
@@ -230,9 +244,15 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
         bad[r] = false;
 #pragma unroll
         for (int d = 0; d < D; ++d) {
-            x[r][d] = p < P ? pos[d * P + p] : 0.0;
-            bad[r] = bad[r] || isnan(x[r][d]);
-            s += fabs(x[r][d]);
+            const double x = p < P ? pos[d * P + p] : 0.0;
+            bad[r] = bad[r] || isnan(x);
+            s += fabs(x);
+            if (d == 0) {
+                x0[r] = x;
+            } else {
+                xf[r][d - 1] = factor_of(x);
+                if (!factor_in_range(x) && !isnan(x)) xabs = __longlong_as_double(0x7ff0000000000000ll);
+            }
         }
         xabs = fmax(xabs, s);
 #pragma unroll
@@ -265,11 +285,15 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
 #pragma unroll 1
         for (int m = 0; m < tm; ++m) {
             const double2 *mr = reinterpret_cast<const double2 *>(rc + m * kRecStaged);
-            const double2 q0 = mr[0], q1 = mr[1];
-            const double k[3] = {q0.x, q0.y, q1.x};
-            const float kb = __int_as_float(__double2loint(q1.y));
+            const float kb = __int_as_float(__double2loint(rc[m * kRecStaged + R_KABS]));
             if (!LIBM && kb * xbound < kFastPhase) {
-                const double2 q2 = mr[2];
+                const double2 q0 = mr[0], q2 = mr[2];
+                double2 q1 = make_double2(0.0, 0.0);
+                if (D > 1) q1 = mr[1];
+                const Factor kf[2] = {{static_cast<uint32_t>(__double2loint(q0.y)), static_cast<uint32_t>(__double2hiint(q0.y)),
+                                       static_cast<uint32_t>(__double2loint(q1.y))},
+                                      {static_cast<uint32_t>(__double2loint(q1.x)), static_cast<uint32_t>(__double2hiint(q1.x)),
+                                       static_cast<uint32_t>(__double2hiint(q1.y))}};
                 const uint64_t beta = static_cast<uint64_t>(__double_as_longlong(q2.x));
                 double av[3] = {q2.y, 0.0, 0.0};
                 if (INC) {
@@ -279,7 +303,11 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
                 }
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
-                    const int64_t c = cos_fixed(turn_fraction(phase_of<D>(k, x[r])) + beta, &sm.tab);
+                    // as phase_of
+                    double ph = __dmul_rn(q0.x, x0[r]);
+#pragma unroll
+                    for (int d = 1; d < D; ++d) ph = __dadd_rn(ph, rn_product(kf[d - 1], xf[r][d - 1]));
+                    const int64_t c = cos_fixed(turn_fraction(ph) + beta, &sm.tab);
                     const int32_t ch = static_cast<int32_t>(c >> 32);
                     const int32_t c0 = static_cast<int32_t>(static_cast<uint32_t>(c) >> 1);
 #pragma unroll
@@ -292,10 +320,15 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
             } else {
                 const double *ex = rec + (t0 + m) * kRec;
                 const double z1 = ex[R_Z1], z2 = ex[R_Z2];
+                const double k[3] = {ex[R_K0], ex[R_K1], ex[R_K2]};
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
+                    const int64_t p = p0 + r * kThreads;
+                    double x[D];
+#pragma unroll
+                    for (int d = 0; d < D; ++d) x[d] = p < P ? pos[d * P + p] : 0.0;
                     double sn, cs;
-                    sincos(phase_of<D>(k, x[r]), &sn, &cs);
+                    sincos(phase_of<D>(k, x), &sn, &cs);
                     const double z12 = __dadd_rn(__dmul_rn(z1, cs), __dmul_rn(z2, sn));
 #pragma unroll
                     for (int i = 0; i < NOUT; ++i) {
@@ -475,8 +508,13 @@ int dispatch_plain(int R, bool incompr, bool libm, int64_t dim, dim3 grid, cudaS
 }
 
 // Launch shape: points per thread R and mode splits S (of mps modes, a
-// multiple of the group of 32), by the time of the busiest SM: its blocks'
-// point*modes, a fixed cost per block, and what the partial sums cost.
+// multiple of the group of 32), by the time of the busiest SM.  Measured on
+// GB300: a point*mode keeps a quarter of an SM for 195, 250 and 295 clocks a warp
+// in 1, 2 and 3 dimensions (280 and 350 for vectors) at R = 2, 7 % more at R = 1
+// and 3 % more at R = 4; a warp alone takes 2.2 times that per mode and point,
+// so an SM wants more than two blocks.  Small calls want the splits that give
+// them (1,000 2-D points x 1000 modes: 262 us with 2 splits at R = 2, 31 us with
+// 32 at R = 1), large ones whole waves.
 struct PlainShape {
     int R;
     int64_t bx, S, mps;
@@ -484,20 +522,17 @@ struct PlainShape {
 PlainShape plain_shape(int64_t P, int64_t chunk, int64_t dim, int64_t nout, int sms, bool libm) {
     PlainShape best{4, (P + 4 * kThreads - 1) / (4 * kThreads), 1, (chunk + kGroup - 1) / kGroup * kGroup};
     double best_cost = 1e300;
-    // clocks a warp holds its quarter of the SM per point*mode: 34 for each
-    // FP64 instruction of a phase and half of the integer work beside it
-    const double pm = libm ? 2000.0 : std::max(68.0 * (2.0 * dim - 1.0), 130.0);
+    const double base = libm ? 2000.0 : nout > 1 ? (dim == 3 ? 350.0 : 280.0) : dim == 1 ? 195.0 : dim == 2 ? 250.0 : 295.0;
+    const int64_t groups = std::max<int64_t>(1, (chunk + kGroup - 1) / kGroup);
     for (int R : {4, 2, 1}) {
         if (libm && R != 4) continue;
+        const double pm = base * (R == 1 ? 1.07 : R == 2 ? 1.0 : 1.03);
         const int64_t bx = (P + kThreads * R - 1) / (kThreads * R);
-        const int64_t groups = std::max<int64_t>(1, (chunk + kGroup - 1) / kGroup);
-        for (int64_t per = groups; per >= 1; --per) {
-            // only the group counts that some split count needs
-            const int64_t S = (groups + per - 1) / per;
-            if (S > 64) break;
-            if (per > 1 && (groups + per - 2) / (per - 1) == S) continue;   // a smaller share, same S
+        for (int64_t S = 1; S <= 64 && S <= groups; ++S) {
+            const int64_t per = (groups + S - 1) / S;
+            if ((groups + per - 1) / per != S) continue;       // fewer splits of the same share
             const double on_sm = std::ceil(static_cast<double>(bx) * S / sms);
-            double cost = on_sm * (per * kGroup * R * pm + 1500.0);
+            double cost = per * kGroup * std::max(on_sm, 2.2) * R * pm;
             if (S > 1) cost += 4000.0 + static_cast<double>(S) * nout * P * 8.0 / 2000.0;
             if (cost < best_cost) {
                 best_cost = cost;
@@ -505,7 +540,6 @@ PlainShape plain_shape(int64_t P, int64_t chunk, int64_t dim, int64_t nout, int 
             }
         }
     }
-    if (chunk == 0) best.S = 1;
     return best;
 }
 
@@ -766,7 +800,7 @@ int batch_plain_launch(int R, int blocks, const BatchItem *items, const BatchUni
 // plain kernel live in one fixed array compiled into the library, so a call
 // allocates nothing; the caller passes the inputs and the output as usual.
 //
-// The array (144 KiB of mode records, enough for 1024 modes) is held on every GPU that loads the library until the process
+// The array (160 KiB of mode records, enough for 1024 modes) is held on every GPU that loads the library until the process
 // exits.  All calls share it and it keeps the last call's contents; every
 // call rewrites the part it reads, so nothing has to start at zero.  Calls
 // whose kernels overlap on the GPU (different streams, no ordering between

@@ -196,7 +196,7 @@ int gsc_summate_dev(const double *cov, const double *z1, const double *z2,
  * that cannot block in the driver's allocator, a plug-in host that hands out
  * memory only from its arena.  The call allocates nothing: the plain FP64
  * kernel's mode records live in a fixed array inside the library
- * (144 KiB, held on every GPU that loads the library until exit), so
+ * (160 KiB, held on every GPU that loads the library until exit), so
  * a call takes at most 1024 modes and returns GSC_ERR_INVALID beyond that.
  * Inputs and output are the caller's device arrays, as for gsc_summate_dev;
  * dim in {1, 2, 3}; forms AUTO or PLAIN_F64 only.  The first call on a
