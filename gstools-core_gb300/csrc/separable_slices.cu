@@ -169,8 +169,8 @@ __device__ __forceinline__ int mode_shift(const SlMode &m, int ew) { return m.am
 // the exponent of 2^23 is its value as a float, one multiply-add takes the
 // offset out and scales it, and the upper halves of two floats are the pair.
 __device__ __forceinline__ void digits6(int64_t re, int64_t im, uint32_t (&w)[kSlices]) {
-    // 256 in each of digits 1 .. 5 (units 2^43, 2^34, 2^25, 2^16, 2^7) and half a unit of the last
-    constexpr int64_t off = (int64_t(256) << 43) + (int64_t(256) << 34) + (int64_t(256) << 25) +
+    // 256 in each digit (units 2^52, 2^43, 2^34, 2^25, 2^16, 2^7) and half a unit of the last
+    constexpr int64_t off = (int64_t(256) << 52) + (int64_t(256) << 43) + (int64_t(256) << 34) + (int64_t(256) << 25) +
                             (int64_t(256) << 16) + (int64_t(256) << 7) + 64;
     const uint64_t a = static_cast<uint64_t>(re + off), b = static_cast<uint64_t>(im + off);
     const uint32_t ah = static_cast<uint32_t>(a >> 32), al = static_cast<uint32_t>(a);
@@ -179,8 +179,7 @@ __device__ __forceinline__ void digits6(int64_t re, int64_t im, uint32_t (&w)[kS
         return fmaf(__uint_as_float(0x4B000000u | field), unit, -8388864.0f * unit);   // (field - 256) unit
     };
     auto pack = [](float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); };
-    w[0] = pack(lift(static_cast<uint32_t>((static_cast<int32_t>(ah) >> 20) + 256), 0x1p-8f),
-                lift(static_cast<uint32_t>((static_cast<int32_t>(bh) >> 20) + 256), 0x1p-8f));
+    w[0] = pack(lift(ah >> 20, 0x1p-8f), lift(bh >> 20, 0x1p-8f));
     w[1] = pack(lift((ah >> 11) & 511u, 0x1p-17f), lift((bh >> 11) & 511u, 0x1p-17f));
     w[2] = pack(lift((ah >> 2) & 511u, 0x1p-26f), lift((bh >> 2) & 511u, 0x1p-26f));
     w[3] = pack(lift(__funnelshift_r(al, ah, 25) & 511u, 0x1p-35f),
@@ -293,10 +292,13 @@ __device__ __forceinline__ int64_t dot_fixed(Word2 a, Word2 b, Word2 c, Word2 d)
 }
 
 // F digits of a slab: grid (2 * row tiles, k-blocks), a thread per row and
-// chunk of four modes.  Bound by the integer pipes (about 600 instructions a
-// thread) and by its stores, 12 bytes per real element.
+// chunk of four modes.  Bound by the integer pipes (about 550 instructions a
+// thread) and by its stores, 12 bytes per real element.  Five blocks per SM
+// (48 registers): with fewer registers it spills, with more it hides less (24,000
+// rows x 1000 modes: 157 us unbounded, 135 at 5 blocks, 172 at 6; two rows per
+// thread, which share s, 139).
 constexpr int kSliceThreads = 256;
-__global__ void __launch_bounds__(kSliceThreads) sl_slice_kernel(SlTab t) {
+__global__ void __launch_bounds__(kSliceThreads, 5) sl_slice_kernel(SlTab t) {
     if (t.words[0]) return;
     const int c = threadIdx.x & 3, r = (blockIdx.x & 1) * 64 + (threadIdx.x >> 2);
     const int kb = blockIdx.y;
@@ -329,10 +331,12 @@ __global__ void __launch_bounds__(kSliceThreads) sl_slice_kernel(SlTab t) {
 struct SlGemm {
     const unsigned char *f, *g;
     int kb, n_tiles;               // k-blocks of the segment, column tiles
-    int splits;                    // CTAs per tile, each a share of the k-blocks
+    int splits;                    // units per tile, each a share of the k-blocks
+    int64_t units;
     int64_t row0, rows_total, P;   // slab's first row; rows of the output; points per component
     int nn, ncn;                   // columns per component, columns
-    double *out;                   // (ncomp, rows, nn); split s of the tile at out + s * split_stride
+    double *out;                   // (ncomp, rows, nn), whole tiles
+    int64_t *part;                 // splits: the integer totals, split s at part + s * split_stride
     int64_t split_stride;
     int accumulate;                // add to the output (later segments)
     int finer;                     // integer totals in units of 2^-(50 + finer)
@@ -341,14 +345,16 @@ struct SlGemm {
 };
 
 // Shared memory: a ring of slots, one slice of F and of G each (the six slices
-// of a k-block in order).  16 slots of 14 KB hold 2.7 k-blocks of 96 columns.
+// of a k-block in order).  14 slots of 14 KB hold 2.3 k-blocks of 96 columns.
 template <int NT>
 struct SlLayout {
     static constexpr int G_BYTES = NT * 64;
     static constexpr int SLOT = kSliceF + G_BYTES;
-    static constexpr int SLOTS = (232448 - 1024 - 512) / SLOT < 24 ? (232448 - 1024 - 512) / SLOT : 24;
-    static constexpr int DATA = SLOTS * SLOT;
-    static constexpr size_t SMEM = DATA + 512 + 1024;
+    static constexpr int EPI_BYTES = 8 * 32 * 9 * 8;    // a worker warp's 32 rows x 8 columns, padded
+    static constexpr int ROOM = 232448 - 1024 - 512 - EPI_BYTES;
+    static constexpr int SLOTS = ROOM / SLOT < 24 ? ROOM / SLOT : 24;
+    static constexpr int DATA = SLOTS * SLOT;           // the ring, then the epilogue's rows, then barriers
+    static constexpr size_t SMEM = DATA + EPI_BYTES + 512 + 1024;
     static constexpr int HC = NT / 2;      // columns per worker half
     static_assert(SLOT % 1024 == 0, "slots keep the swizzle's alignment");
     // with at most 24 slots, k-block i + 4 is not copied before k-block i has been
@@ -356,7 +362,6 @@ struct SlLayout {
     static_assert(SLOTS >= 12 && SLOTS <= 24, "two k-blocks at least, four at most");
     static_assert((8 + 2 * kAccs + 1) * 8 + 16 <= 512, "barriers");
     static_assert(NT % 16 == 0 && NT <= kAccCols && HC % 8 == 0, "tile width");
-    static_assert(8 * 32 * 17 * 8 <= DATA, "epilogue buffers");
 };
 
 // What a unit of each accumulator counts in a 64-bit total of units 2^-(50 + finer).
@@ -403,13 +408,35 @@ __device__ __forceinline__ void drain_acc(int64_t (&acc)[HC], uint32_t taddr, co
     }
 }
 
-// One tile of 128 rows x NT columns, k-blocks of one split.  Per k-block 52 MMAs
-// of 128 x NT x 16 beside 1.7 drained accumulators.  The products are issued by
-// F slice, the slice kept in the collector buffer for its products (an MMA of 96
-// columns takes 56 clocks when it reads both operands and 48 when it keeps A; 52
-// and 41 for 80), except those of level 3, which come last: its accumulator is
-// drained every second k-block, and this way the drain overlaps the other
-// levels' MMAs of the next one.
+__device__ __noinline__ double scaled_total_small(int64_t t, int e) { return ldexp(static_cast<double>(t), e); }
+
+// t 2^e for an integer total, rounded to nearest even, by integer instructions (a
+// conversion is an FP64 instruction: 16 clocks of an SM for a warp's).  The
+// subnormal results' path is a call, so that it is not run in advance.
+__device__ __forceinline__ double scaled_total(int64_t t, int e) {
+    if (t == 0) return 0.0;
+    const uint64_t mag = static_cast<uint64_t>(t < 0 ? -t : t);
+    const int lz = __clzll(static_cast<long long>(mag));
+    const uint64_t m = mag << lz;                    // leading bit at 63
+    const int x = 63 - lz + e;                       // the value is 1.m 2^x
+    if (x < -1020) return scaled_total_small(t, e);
+    const uint64_t inc = ((m & 0x7ffu) + 0x3ffu + ((m >> 11) & 1u)) >> 11;
+    // the leading bit adds one to the exponent field
+    const uint64_t bits = (m >> 11) + inc + (static_cast<uint64_t>(x + 1022) << 52);
+    return __longlong_as_double(static_cast<long long>(bits | (t < 0 ? uint64_t(1) << 63 : 0)));
+}
+
+// Tiles of 128 rows x NT columns.  One CTA per SM walks units (a tile, or one
+// split of its k-blocks); the copies and MMAs of a unit follow those of the one
+// before at once, while the workers still write that one out: its sums are in
+// their registers.
+//
+// Per k-block 52 MMAs of 128 x NT x 16 beside 1.7 drained accumulators.  The
+// products run in three groups, levels 0 to 2, level 3, tail, so that an
+// accumulator that was just drained is needed again one group later at the
+// earliest, and within a group by F slice, which the collector buffer keeps for
+// its products (an MMA of 96 columns takes 56 clocks when it reads both operands
+// and 48 when it keeps A; 52 and 41 for 80).
 template <int NT>
 __global__ void __launch_bounds__(kThreads, 1) sl_gemm_kernel(const SlGemm p) {
     using L = SlLayout<NT>;
@@ -417,8 +444,8 @@ __global__ void __launch_bounds__(kThreads, 1) sl_gemm_kernel(const SlGemm p) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::DATA);   // [4] copies of k-block i at i % 4 -> MMA
-    uint64_t *kdone = full + 4;                  // [4] MMA commit of k-block i at i % 4 -> copies
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::DATA + L::EPI_BYTES);   // [4] copies -> MMA
+    uint64_t *kdone = full + 4;                  // [4] MMA commit of a k-block -> copies
     uint64_t *acc_full = kdone + 4;              // [5] MMA commit -> workers
     uint64_t *acc_empty = acc_full + kAccs;      // [5] workers -> MMA (8 arrivals)
     uint64_t *drain = acc_empty + kAccs;
@@ -426,12 +453,21 @@ __global__ void __launch_bounds__(kThreads, 1) sl_gemm_kernel(const SlGemm p) {
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int u = static_cast<int>(blockIdx.x);
-    const int part = u % p.splits, tile = u / p.splits;
-    const int nt = tile % p.n_tiles;
-    const int64_t mt = tile / p.n_tiles;
-    const int kbeg = static_cast<int>(static_cast<int64_t>(part) * p.kb / p.splits);
-    const int KB = static_cast<int>(static_cast<int64_t>(part + 1) * p.kb / p.splits) - kbeg;
+    // a unit's tile and k-blocks
+    struct Unit {
+        int nt, part, kbeg, kb;
+        int64_t mt;
+    };
+    auto unit_at = [&](int64_t u) -> Unit {
+        Unit x;
+        x.part = static_cast<int>(u % p.splits);
+        const int64_t tile = u / p.splits;
+        x.nt = static_cast<int>(tile % p.n_tiles);
+        x.mt = tile / p.n_tiles;
+        x.kbeg = static_cast<int>(static_cast<int64_t>(x.part) * p.kb / p.splits);
+        x.kb = static_cast<int>(static_cast<int64_t>(x.part + 1) * p.kb / p.splits) - x.kbeg;
+        return x;
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < 4; ++s) {
@@ -455,94 +491,152 @@ __global__ void __launch_bounds__(kThreads, 1) sl_gemm_kernel(const SlGemm p) {
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
+    // k-blocks are counted through all units of the CTA: k-block `it` uses
+    // barriers it % 4 and the ring slots from 6 it on
     if (warp == kCopyWarp) {
         if (elect_one()) {
-            const unsigned char *fb = p.f + (mt * p.kb + kbeg) * (kSlices * kSliceF);
-            const unsigned char *gb = p.g + (static_cast<int64_t>(nt) * p.kb + kbeg) * (kSlices * L::G_BYTES);
-            int issued = 0;                // k-blocks whose barrier has been armed
             bool ok = true;
-            for (int i = 0, q = 0; i < KB && ok; ++i) {
-                for (int s = 0; s < kSlices; ++s, ++q) {
-                    if (q >= L::SLOTS) {       // the k-block that last used the slot has been multiplied
-                        const int k = (q - L::SLOTS) / kSlices;
-                        ok = mbar_wait(&kdone[k & 3], (k >> 2) & 1, abort_flag, p.status, kErrTimeoutEmpty);
-                        if (!ok) break;
+            int it = 0, slot = 0;
+            for (int64_t u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
+                const Unit x = unit_at(u);
+                const unsigned char *fb = p.f + (x.mt * p.kb + x.kbeg) * (kSlices * kSliceF);
+                const unsigned char *gb =
+                    p.g + (static_cast<int64_t>(x.nt) * p.kb + x.kbeg) * (kSlices * L::G_BYTES);
+                for (int i = 0; i < x.kb && ok; ++i, ++it) {
+                    for (int s = 0; s < kSlices; ++s) {
+                        const int q = it * kSlices + s - L::SLOTS;
+                        if (q >= 0) {          // the k-block that last used the slot has been multiplied
+                            const int k = q / kSlices;
+                            ok = mbar_wait(&kdone[k & 3], (k >> 2) & 1, abort_flag, p.status, kErrTimeoutEmpty);
+                            if (!ok) break;
+                        }
+                        if (s == 0) mbar_arrive_expect_tx(&full[it & 3], kSlices * L::SLOT);
+                        unsigned char *dst = smem + slot * L::SLOT;
+                        bulk_copy_g2s(dst, fb, kSliceF, &full[it & 3]);
+                        bulk_copy_g2s(dst + kSliceF, gb, L::G_BYTES, &full[it & 3]);
+                        fb += kSliceF;
+                        gb += L::G_BYTES;
+                        slot = slot + 1 == L::SLOTS ? 0 : slot + 1;
                     }
-                    if (s == 0) {
-                        mbar_arrive_expect_tx(&full[i & 3], kSlices * L::SLOT);
-                        issued = i + 1;
-                    }
-                    unsigned char *dst = smem + (q % L::SLOTS) * L::SLOT;
-                    bulk_copy_g2s(dst, fb + static_cast<int64_t>(q) * kSliceF, kSliceF, &full[i & 3]);
-                    bulk_copy_g2s(dst + kSliceF, gb + static_cast<int64_t>(q) * L::G_BYTES, L::G_BYTES,
-                                  &full[i & 3]);
                 }
             }
-            // on abort the copies in flight land before the block ends; a k-block that
-            // was cut short never completes its barrier, and that wait runs out
+            // on abort the copies in flight land before the block ends; a k-block
+            // that was cut short never completes its barrier, and that wait runs out
             if (*abort_flag)
-                for (int i = issued > 4 ? issued - 4 : 0; i < issued; ++i)
+                for (int i = it > 3 ? it - 3 : 0; i < it; ++i)
                     mbar_wait_drain(&full[i & 3], (i >> 2) & 1, p.status);
         }
     } else if (warp == kMmaWarp) {
         if (elect_one()) {
+            // Little time may pass between two MMAs: the unit holds only a few
+            // that were issued ahead.  So what a k-block needs is prepared between
+            // the MMAs of the one before, a piece at a time, and accumulators are
+            // waited for one by one, each right before its first product.
             constexpr uint32_t idesc = idesc_f16(kTileRows, NT, true);
             bool ok = true;
-            for (int i = 0; i < KB; ++i) {
-                ok = mbar_wait(&full[i & 3], (i >> 2) & 1, abort_flag, p.status, kErrTimeoutFull);
-                // accumulators drained since the last k-block start again from zero
-                uint32_t keep[kAccs];
+            int it = 0, slot = 0;
+            uint32_t phase[kAccs] = {0, 0, 0, 0, 0};   // drains handed to the workers so far
+            int left[kAccs];                           // k-blocks until the next drain
+            uint32_t keep[kAccs];                      // 0: the accumulator starts again from zero
+            uint64_t fd[kSlices], gd[kSlices], nf[kSlices], ng[kSlices];
+            auto next_slot = [&](int s) {
+                const uint32_t at = smem_u32(smem + slot * L::SLOT);
+                nf[s] = desc_k_sw64(at);
+                ng[s] = desc_k_sw64(at + kSliceF);
+                slot = slot + 1 == L::SLOTS ? 0 : slot + 1;
+            };
 #pragma unroll
-                for (int a = 0; a < kAccs; ++a) {
-                    const int per = drain_period(a);
-                    keep[a] = i % per != 0;
-                    if (a != 3 && !keep[a] && i > 0 && ok)
-                        ok = mbar_wait(&acc_empty[a], (i / per - 1) & 1, abort_flag, p.status, kErrTimeoutAcc);
-                }
+            for (int s = 0; s < kSlices; ++s) next_slot(s);
+            bool ready = false;                        // the k-block's copies have been waited for
+            int64_t u = blockIdx.x;
+            int KB = u < p.units ? unit_at(u).kb : 0, i = 0;
+            while (KB > 0) {
+                if (!ready) ok = mbar_wait(&full[it & 3], (it >> 2) & 1, abort_flag, p.status, kErrTimeoutFull);
                 if (!ok) break;
                 tc_fence_after();
-                uint64_t fd[kSlices], gd[kSlices];
 #pragma unroll
                 for (int s = 0; s < kSlices; ++s) {
-                    const uint32_t at = smem_u32(smem + ((i * kSlices + s) % L::SLOTS) * L::SLOT);
-                    fd[s] = desc_k_sw64(at);
-                    gd[s] = desc_k_sw64(at + kSliceF);
+                    fd[s] = nf[s];
+                    gd[s] = ng[s];
                 }
-                // (the K step of 16 adds 32 bytes to an address: 2 in the descriptor)
+                if (i == 0) {
 #pragma unroll
-                for (int x = 0; x < kSlices; ++x) {
-#pragma unroll
-                    for (int kk = 0; kk < 2; ++kk) {
-                        bool filled = false;
-#pragma unroll
-                        for (int y = 0; y < kSlices; ++y) {
-                            const int l = x + y;
-                            if (l == 3 || l > 6) continue;
-                            const int a = l < kTail ? l : kTail;
-                            const bool opens = x == 0 && kk == 0 && y <= kTail;   // first product of its accumulator
-                            const uint32_t d = tmem + a * kAccCols, acc = opens ? keep[a] : 1u;
-                            if (filled) mma_f16_ss_keep<true>(d, fd[x] + 2 * kk, gd[y] + 2 * kk, idesc, acc);
-                            else mma_f16_ss_keep<false>(d, fd[x] + 2 * kk, gd[y] + 2 * kk, idesc, acc);
-                            filled = true;
-                        }
+                    for (int a = 0; a < kAccs; ++a) {
+                        left[a] = drain_period(a);
+                        keep[a] = 0;
                     }
-                    if (x < 3 && ((i + 1) % drain_period(x) == 0 || i == KB - 1)) mma_commit(&acc_full[x]);
-                    if (x == kSlices - 1 && ((i + 1) % drain_period(kTail) == 0 || i == KB - 1))
-                        mma_commit(&acc_full[kTail]);
                 }
-                if (!keep[3] && i > 0) {
-                    ok = mbar_wait(&acc_empty[3], (i / drain_period(3) - 1) & 1, abort_flag, p.status, kErrTimeoutAcc);
-                    if (!ok) break;
-                    tc_fence_after();
+                const bool last = i == KB - 1;
+                // before an accumulator's first product: it may start again once the
+                // workers have read it
+                auto open = [&](int a) {
+                    if (!keep[a] && phase[a] > 0 && ok) {
+                        ok = mbar_wait(&acc_empty[a], (phase[a] - 1) & 1, abort_flag, p.status, kErrTimeoutAcc);
+                        tc_fence_after();
+                    }
+                };
+                // after its last product: drained when its period or the unit ends
+                auto close = [&](int a) {
+                    keep[a] = 1;
+                    if (--left[a] == 0 || last) {
+                        mma_commit(&acc_full[a]);
+                        ++phase[a];
+                        left[a] = drain_period(a);
+                        keep[a] = 0;
+                    }
+                };
+                // products (x, y) of F slice x with lo <= x + y <= hi into accumulator
+                // min(x + y, tail); (the K step of 16 adds 32 bytes to an address, 2 in a
+                // descriptor)
+                auto group = [&](auto lo_, auto hi_, auto &&between) {
+                    constexpr int lo = decltype(lo_)::value, hi = decltype(hi_)::value;
+                    int n = 0;                         // a constant at every use once unrolled
+#pragma unroll
+                    for (int x = 0; x < kSlices; ++x)
+#pragma unroll
+                        for (int kk = 0; kk < 2; ++kk) {
+                            bool filled = false;
+#pragma unroll
+                            for (int y = 0; y < kSlices; ++y) {
+                                const int l = x + y;
+                                if (l < lo || l > hi) continue;
+                                const int a = l < kTail ? l : kTail;
+                                const bool opens = x == 0 && kk == 0 && y == a;
+                                if (opens) open(a);
+                                const uint32_t d = tmem + a * kAccCols, acc = opens ? keep[a] : 1u;
+                                if (filled) mma_f16_ss_keep<true>(d, fd[x] + 2 * kk, gd[y] + 2 * kk, idesc, acc);
+                                else mma_f16_ss_keep<false>(d, fd[x] + 2 * kk, gd[y] + 2 * kk, idesc, acc);
+                                filled = true;
+                                between(n);
+                                ++n;
+                            }
+                        }
+                };
+                group(std::integral_constant<int, 0>{}, std::integral_constant<int, 2>{}, [&](int n) {
+                    if (n == 9) close(0);              // products 0, 3 are level 0's, 1, 4, 6, 8 level 1's
+                    if (n == 10) close(1);
+                });
+                close(2);
+                group(std::integral_constant<int, 3>{}, std::integral_constant<int, 3>{}, [](int) {});
+                close(3);
+                ready = false;
+                group(std::integral_constant<int, kTail>{}, std::integral_constant<int, 6>{}, [&](int n) {
+#pragma unroll
+                    for (int s = 0; s < kSlices; ++s)
+                        if (n == 3 + 2 * s) next_slot(s);
+                    if (n == 20 && !last)
+                        ready = mbar_test_wait(&full[(it + 1) & 3], ((it + 1) >> 2) & 1);
+                });
+                close(kTail);
+                mma_commit(&kdone[it & 3]);
+                ++it;
+                ++i;
+                if (last) {
+                    u += gridDim.x;
+                    KB = u < p.units ? unit_at(u).kb : 0;
+                    i = 0;
                 }
-#pragma unroll
-                for (int x = 0; x <= 3; ++x)
-#pragma unroll
-                    for (int kk = 0; kk < 2; ++kk)
-                        mma_f16_ss(tmem + 3 * kAccCols, fd[x] + 2 * kk, gd[3 - x] + 2 * kk, idesc,
-                                   (x == 0 && kk == 0) ? keep[3] : 1u);
-                if ((i + 1) % drain_period(3) == 0 || i == KB - 1) mma_commit(&acc_full[3]);
-                mma_commit(&kdone[i & 3]);
+                if (!ok) break;
             }
             if (!ok) {
                 mma_commit(drain);
@@ -553,69 +647,70 @@ __global__ void __launch_bounds__(kThreads, 1) sl_gemm_kernel(const SlGemm p) {
         // ---- workers ---------------------------------------------------------
         const int q = warp & 3, h = warp >> 2;
         const uint32_t taddr = tmem + (static_cast<uint32_t>(32 * q) << 16) + L::HC * h;
-        int64_t acc[L::HC];
-#pragma unroll
-        for (int c = 0; c < L::HC; ++c) acc[c] = 0;
+        int64_t *tr = reinterpret_cast<int64_t *>(smem + L::DATA) + warp * (32 * 9);
         Units units;
         units.zero = 1 << (2 + p.finer);
         units.one = 1 << (25 + p.finer);
         units.two = 1 << (16 + p.finer);
         units.three = 1 << (7 + p.finer);
         units.tail = ldexpf(1.0f, 50 + p.finer);
+        const int ew = top_exponent(p.words[1]);
+        int drains[kAccs] = {0, 0, 0, 0, 0};
         bool ok = true;
-        // a drain is taken by the whole warp: the barrier counts once every lane has passed it
-        auto take = [&](auto level, int i) {
-            constexpr int A = decltype(level)::value;
-            constexpr int per = drain_period(A);
-            if (!ok || !((i + 1) % per == 0 || i == KB - 1)) return;
-            const bool got = mbar_wait(&acc_full[A], (i / per) & 1, abort_flag, p.status, kErrTimeoutAcc);
-            ok = __all_sync(0xffffffffu, got);
-            if (!ok) return;
-            tc_fence_after();
-            drain_acc<A>(acc, taddr + A * kAccCols, units);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[A]);
-        };
-        for (int i = 0; i < KB && ok; ++i) {
-            take(std::integral_constant<int, 0>{}, i);
-            take(std::integral_constant<int, 1>{}, i);
-            take(std::integral_constant<int, 2>{}, i);
-            take(std::integral_constant<int, kTail>{}, i);
-            take(std::integral_constant<int, 3>{}, i);
-        }
-        // ---- epilogue: every MMA and copy has completed, the slots are free ----
-        // 16 columns at a time are turned around in shared memory, so that half
-        // a warp writes 128 consecutive bytes of a row
-        if (ok) {
-            asm volatile("bar.sync 1, 256;" ::: "memory");      // the last drains of all workers are past
-            double *tr = reinterpret_cast<double *>(smem) + warp * (32 * 17);
-            const int ew = top_exponent(p.words[1]);
-            const int64_t rq = p.row0 + mt * kTileRows + 32 * q;
-            const int rows = static_cast<int>(min(static_cast<int64_t>(32), p.rows_total - rq));
-            const int n0 = nt * NT + L::HC * h;
+        for (int64_t u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
+            const Unit x = unit_at(u);
+            int64_t acc[L::HC];
 #pragma unroll
-            for (int c0 = 0; c0 < L::HC; c0 += 16) {
-                constexpr int W = 16;
-#pragma unroll
-                for (int c = 0; c < W; ++c) {
-                    if (c0 + c >= L::HC) break;
-                    tr[lane * 17 + c] = static_cast<double>(acc[c0 + c]);
-                }
+            for (int c = 0; c < L::HC; ++c) acc[c] = 0;
+            // a drain is taken by the whole warp: the barrier counts once every lane has passed it
+            auto take = [&](auto level, int i) {
+                constexpr int A = decltype(level)::value;
+                if (!ok || !((i + 1) % drain_period(A) == 0 || i == x.kb - 1)) return;
+                const bool got = mbar_wait(&acc_full[A], drains[A] & 1, abort_flag, p.status, kErrTimeoutAcc);
+                ++drains[A];
+                ok = __all_sync(0xffffffffu, got);
+                if (!ok) return;
+                tc_fence_after();
+                drain_acc<A>(acc, taddr + A * kAccCols, units);
+                tc_fence_before();
                 __syncwarp();
-                const int c = lane & 15, col = n0 + c0 + c;
-                if (c0 + c < L::HC && col < p.ncn) {
+                if (lane == 0) mbar_arrive(&acc_empty[A]);
+            };
+            for (int i = 0; i < x.kb && ok; ++i) {
+                take(std::integral_constant<int, 0>{}, i);
+                take(std::integral_constant<int, 1>{}, i);
+                take(std::integral_constant<int, 2>{}, i);
+                take(std::integral_constant<int, 3>{}, i);
+                take(std::integral_constant<int, kTail>{}, i);
+            }
+            if (!ok) break;
+            // ---- the unit's output: 8 columns at a time are turned around in
+            // shared memory, so that a quarter of a warp writes 64 consecutive
+            // bytes.  Splits leave their integers: their sum is exact, and the
+            // conversion (an FP64 instruction) waits for it
+            const int64_t rq = p.row0 + x.mt * kTileRows + 32 * q;
+            const int rows = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(32), p.rows_total - rq)));
+            const int n0 = x.nt * NT + L::HC * h;
+#pragma unroll
+            for (int c0 = 0; c0 < L::HC; c0 += 8) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) tr[lane * 9 + c] = acc[c0 + c];
+                __syncwarp();
+                const int c = lane & 7, col = n0 + c0 + c;
+                if (col < p.ncn) {
                     const int comp = col / p.nn;
-                    const int g = p.words[2 + comp] > 0 ? top_exponent(p.words[2 + comp]) : 0;
-                    const int e = ew + g - 50 - p.finer;
-                    double *o = p.out + part * p.split_stride + comp * p.P + (col - comp * p.nn);
-                    for (int r = lane >> 4; r < rows; r += 2) {
-                        double v = tr[r * 17 + c];
-                        // |v| is 0 or in [1, 2^63): a power of two by its exponent bits
-                        if (e < -960) v = ldexp(v, e);
-                        else if (v != 0.0) v = __hiloint2double(__double2hiint(v) + e * (1 << 20), __double2loint(v));
-                        double *dst = o + (rq + r) * p.nn;
-                        *dst = p.accumulate ? *dst + v : v;
+                    const int64_t at = comp * p.P + (col - comp * p.nn);
+                    if (p.part) {
+                        int64_t *o = p.part + x.part * p.split_stride + at + rq * p.nn;
+                        for (int r = lane >> 3; r < rows; r += 4) o[static_cast<int64_t>(r) * p.nn] = tr[r * 9 + c];
+                    } else {
+                        const int e = ew + top_exponent(p.words[2 + comp]) - 50 - p.finer;
+                        double *o = p.out + at + rq * p.nn;
+                        for (int r = lane >> 3; r < rows; r += 4) {
+                            const double v = scaled_total(tr[r * 9 + c], e);
+                            double *dst = o + static_cast<int64_t>(r) * p.nn;
+                            *dst = p.accumulate ? *dst + v : v;
+                        }
                     }
                 }
                 __syncwarp();
@@ -628,15 +723,27 @@ __global__ void __launch_bounds__(kThreads, 1) sl_gemm_kernel(const SlGemm p) {
     if (warp == kMmaWarp) tmem_dealloc(tmem, kTmem);
 }
 
-// out = the splits' partial fields added in order
+// out = the splits' integer totals, added and converted: exact within a segment
+// of modes (segments of `splits` totals each, the last of `last`), one rounding
+// and for later segments one addition each
 __global__ void __launch_bounds__(256)
-sl_reduce_kernel(const double *__restrict__ part, int splits, int64_t n, double *__restrict__ out,
-                 const int *__restrict__ words) {
+sl_reduce_kernel(const int64_t *__restrict__ part, int segs, int splits, int last, int64_t P, int ncomp,
+                 int finer, double *__restrict__ out, const int *__restrict__ words) {
     if (words[0]) return;
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
-    if (i >= n) return;
-    double s = part[i];
-    for (int k = 1; k < splits; ++k) s += part[k * n + i];
+    const int64_t q = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x, n = ncomp * P;
+    if (q >= P) return;
+    const int64_t i = blockIdx.y * P + q;
+    const int e = top_exponent(words[1]) + top_exponent(words[2 + blockIdx.y]) - 50 - finer;
+    double s = 0.0;
+    for (int g = 0; g < segs; ++g) {
+        const int k1 = g == segs - 1 ? last : splits;
+        int64_t t = 0;
+#pragma unroll 4
+        for (int k = 0; k < k1; ++k) t += part[(static_cast<int64_t>(g) * splits + k) * n + i];
+        const double v = scaled_total(t, e);
+        if (g == 0) s = v;
+        else s += v;
+    }
     out[i] = s;
 }
 
@@ -652,9 +759,9 @@ size_t up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // clocks of a k-block's 52 MMAs of 128 x nt x 16: nt / 2 for the multiplies, and
 // 128 bytes of shared memory per clock for the operands: 32 nt, and 4 KB more
-// for the 20 that read F
+// for the 26 that read F
 double kblock_clocks(int nt) {
-    return 20.0 * std::max(nt * 0.5, (4096.0 + 32.0 * nt) / 128.0) + 32.0 * nt * 0.5;
+    return 26.0 * std::max(nt * 0.5, (4096.0 + 32.0 * nt) / 128.0) + 26.0 * nt * 0.5;
 }
 
 }  // namespace
@@ -705,7 +812,7 @@ static SlPlan sl_plan(int64_t rows, int ncn, int64_t n_modes, int64_t out_bytes,
         const int64_t tiles = s.m_tiles * s.n_tiles;
         for (int k = 1; k <= 64 && s.kb / k >= 2; ++k) {
             if (k > 1 && static_cast<int64_t>(k) * s.segs * out_bytes > (int64_t(1) << 30)) break;
-            double c = std::ceil(static_cast<double>(tiles * k) / sms) * (std::ceil(static_cast<double>(s.kb) / k) * kb_clocks + 9000.0);
+            double c = std::ceil(static_cast<double>(tiles * k) / sms) * (std::ceil(static_cast<double>(s.kb) / k) * kb_clocks + 4000.0);
             if (k > 1) c += 4000.0 + (k + 1.0) * out_bytes / 2500.0;
             if (c < least) {
                 least = c;
@@ -772,7 +879,11 @@ int sep_slices_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
     t.g = base + off_g;
     t.f = base + off_f;
     t.rows_total = rows;
-    double *part = reinterpret_cast<double *>(base + off_part);
+    int64_t *part = reinterpret_cast<int64_t *>(base + off_part);
+
+    // |total| <= the modes of a segment <= 2^(12 - finer)
+    int finer = 0;
+    while (finer < kFinest && N <= (kSegModes >> (finer + 1))) ++finer;
 
     GSC_CUDA(cudaMemsetAsync(t.words, 0, kWords * sizeof(int), st));
     {
@@ -825,15 +936,13 @@ int sep_slices_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
             p.status = a.status;
             p.out = a.out;
             p.accumulate = seg > 0;
-            // |total| <= the segment's modes <= 2^(12 - finer)
-            while (p.finer < kFinest && t.nj <= (kSegModes >> (p.finer + 1))) ++p.finer;
+            p.finer = finer;
             if (parts > 0) {
-                p.out = part + static_cast<size_t>(seg) * pl.splits * ncomp * P;
+                p.part = part + static_cast<size_t>(seg) * pl.splits * ncomp * P;
                 p.split_stride = static_cast<int64_t>(ncomp) * P;
-                p.accumulate = 0;
             }
-            const int64_t grid = mts * pl.n_tiles * p.splits;
-            if (grid > 0x7fffffff) return set_error(GSC_ERR_INVALID, "grid too large");
+            p.units = mts * pl.n_tiles * p.splits;
+            const int64_t grid = std::min<int64_t>(p.units, sms);
             TimedLaunch tl(st);
             tl.begin(K_SEP_F64_SLICES);
             if (pl.nt == 96) GSC_TRY(launch_gemm<96>(p, grid, st));
@@ -845,13 +954,12 @@ int sep_slices_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
         }
     }
     if (parts > 0) {
-        // the last segment may be shorter than the splits: its parts are fewer
-        const int last = N - (pl.segs - 1) * kSegModes;
-        const int used = (pl.segs - 1) * pl.splits + std::min(pl.splits, (last + kKbModes - 1) / kKbModes);
-        const int64_t n = static_cast<int64_t>(ncomp) * P;
+        // the last segment may have fewer k-blocks than the splits
+        const int kb_last = (N - (pl.segs - 1) * kSegModes + kKbModes - 1) / kKbModes;
         TimedLaunch tl(st);
         tl.begin(K_SPLIT_REDUCE);
-        sl_reduce_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(part, used, n, a.out, t.words);
+        sl_reduce_kernel<<<dim3(static_cast<unsigned>((P + 255) / 256), ncomp), 256, 0, st>>>(
+            part, pl.segs, pl.splits, std::min(pl.splits, kb_last), P, ncomp, finer, a.out, t.words);
         tl.end();
         GSC_CUDA(cudaGetLastError());
     }
