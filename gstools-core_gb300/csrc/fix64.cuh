@@ -238,10 +238,26 @@ __device__ __forceinline__ double rn_product(const Factor &x, const Factor &y) {
     return __longlong_as_double(static_cast<long long>(r));
 }
 
+// x = f 2^e with |f| in [1/2, 1) for finite x != 0, as frexp gives e (from the
+// exponent field where x is normal; frexp is a long call)
+__device__ __forceinline__ int exponent_of(double x) {
+    const int field = static_cast<int>((static_cast<uint32_t>(__double2hiint(x)) >> 20) & 0x7ffu);
+    if (field != 0) return field - 1022;
+    int e;
+    frexp(x, &e);
+    return e;
+}
+// x 2^n as ldexp(x, n) gives it: a product with the power of two where that is a
+// normal double
+__device__ __forceinline__ double scale_pow2(double x, int n) {
+    if (n >= -1022 && n <= 1023) return x * __hiloint2double((n + 1023) << 20, 0);
+    return ldexp(x, n);
+}
+
 // Finite z1, z2 as z1 + i z2 = amp 2^ez e^{i beta} (amp in [1/2, sqrt 2), or
 // 0): a first angle in FP32, its cosine and sine in 64 bits, then the remaining
 // rotation d (1e-7 rad) from the cross product.  An FP64 atan2 and hypot would
-// be a chain of several microseconds, and less exact.
+// be a longer chain, and less exact.
 __device__ __forceinline__ void mode_angle(double z1, double z2, const CosTable *tab, double *amp,
                                            int *ez, uint64_t *beta) {
     *amp = 0.0;
@@ -249,16 +265,17 @@ __device__ __forceinline__ void mode_angle(double z1, double z2, const CosTable 
     *beta = 0;
     const double zm = fmax(fabs(z1), fabs(z2));
     if (zm == 0.0) return;
-    frexp(zm, ez);
-    const double y1 = ldexp(z1, -*ez), y2 = ldexp(z2, -*ez);
-    const float t = atan2f(static_cast<float>(y2), static_cast<float>(y1)) * 0.15915494f;   // turns
+    *ez = exponent_of(zm);
+    const int64_t f1 = __double2ll_rn(scale_pow2(z1, 62 - *ez)), f2 = __double2ll_rn(scale_pow2(z2, 62 - *ez));
+    const float t = atan2f(static_cast<float>(f2), static_cast<float>(f1)) * 0.15915494f;   // turns
     const uint64_t b = static_cast<uint64_t>(__float2ll_rn(t * 1099511627776.0f)) << 24;
-    const int64_t f1 = __double2ll_rn(y1 * 0x1p62), f2 = __double2ll_rn(y2 * 0x1p62);
     int64_t c, s;
     cis_fine(b + kFineOffset, tab, &c, &s);
     const double along = static_cast<double>(__mul64hi(f1, c) + __mul64hi(f2, s));    // units 2^-60
     const double across = static_cast<double>(__mul64hi(f2, c) - __mul64hi(f1, s));
-    const double d = across / along;
+    // across / along to 2^-45 of it: an FP32 reciprocal and one Newton step
+    const double r0 = static_cast<double>(__frcp_rn(static_cast<float>(along)));
+    const double d = across * fma(fma(-along, r0, 1.0), r0, r0);
     *amp = fma(along, 0.5 * d * d, along) * 0x1p-60;
     *beta = b + static_cast<uint64_t>(__double2ll_rn(d * 2.935890503282001e18));      // 2^64 / 2 pi
 }

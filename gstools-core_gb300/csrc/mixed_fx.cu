@@ -47,6 +47,7 @@
 
 #include "dfturns.cuh"
 #include "internal.h"
+#include "launch.cuh"
 
 namespace gsc {
 namespace {
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(kFxRangeThreads)
 fx_range_kernel(const double *__restrict__ pos, int64_t P, int dim,
                 unsigned long long *__restrict__ part, unsigned long long *maxbits) {
     __shared__ unsigned long long wm[kFxRangeThreads / 32][3];
+    after_previous();
     unsigned long long m[3] = {0ull, 0ull, 0ull};
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < P; i += stride)
@@ -245,6 +247,7 @@ fx_mode_kernel(const double *__restrict__ cov, const double *__restrict__ z1,
                unsigned long long *maxbits, uint32_t *__restrict__ rec, int *range_flag) {
     // the mode's inputs first (they may come over the host link), so that
     // their latency overlaps the reduction of the range words
+    after_previous();
     const int64_t jl = static_cast<int64_t>(blockIdx.x) * kFxModeThreads + threadIdx.x;
     const int64_t j = j0 + jl;
     const bool mine = jl < nc;
@@ -537,6 +540,7 @@ mixed_fx_kernel(const double *__restrict__ pos, int64_t P, const uint32_t *__res
                 int64_t split_stride) {
     constexpr int TILE = R >= 8 ? kFxTile : kFxTile / 2;
     __shared__ __align__(256) uint32_t srec[TILE * kFxRecWords];
+    after_previous();
     const int64_t jb = static_cast<int64_t>(blockIdx.y) * mps;
     const int64_t je = min(nc, jb + mps);
     fx_block<D, R, INC, TILE>(pos, P, static_cast<int64_t>(blockIdx.x) * (kFxThreads * R), rec, jb,
@@ -549,16 +553,9 @@ template <int D, bool INC>
 int launch_fx(int R, dim3 grid, cudaStream_t st, const double *pos, int64_t P, const uint32_t *rec,
               const unsigned long long *maxbits, int64_t nc, int64_t mps, int accumulate,
               double *dst, int64_t sd, int64_t sp, int64_t split_stride) {
-    if (R == 2)
-        mixed_fx_kernel<D, INC, 2><<<grid, kFxThreads, 0, st>>>(pos, P, rec, maxbits, nc, mps,
-                                                                accumulate, dst, sd, sp, split_stride);
-    else if (R == 8)
-        mixed_fx_kernel<D, INC, 8><<<grid, kFxThreads, 0, st>>>(pos, P, rec, maxbits, nc, mps,
-                                                                accumulate, dst, sd, sp, split_stride);
-    else
-        mixed_fx_kernel<D, INC, 4><<<grid, kFxThreads, 0, st>>>(pos, P, rec, maxbits, nc, mps,
-                                                                accumulate, dst, sd, sp, split_stride);
-    GSC_CUDA(cudaGetLastError());
+    const auto fn = R == 2 ? mixed_fx_kernel<D, INC, 2> : R == 8 ? mixed_fx_kernel<D, INC, 8> : mixed_fx_kernel<D, INC, 4>;
+    GSC_CUDA(launch_after(fn, grid, dim3(kFxThreads), 0, st, pos, P, rec, maxbits, nc, mps, accumulate, dst, sd, sp,
+                          split_stride));
     return GSC_OK;
 }
 
@@ -813,12 +810,10 @@ int mixed_fx_run(DeviceCtx &ctx, const PlainArgs &a, int *range_flag, cudaStream
         if (nc <= 0) return GSC_OK;
         TimedLaunch tl(st);
         tl.begin(K_MIXED_MODES);
-        fx_mode_kernel<<<static_cast<unsigned>((nc + kFxModeThreads - 1) / kFxModeThreads),
-                         kFxModeThreads, 0, st>>>(
-            a.cov, a.z1, a.z2, static_cast<int>(dim), N, j0, nc, a.incompr ? 1 : 0, range_part,
-            static_cast<int>(rb), maxbits, rec, range_flag);
+        GSC_CUDA(launch_after(fx_mode_kernel, dim3(static_cast<unsigned>((nc + kFxModeThreads - 1) / kFxModeThreads)),
+                              dim3(kFxModeThreads), 0, st, a.cov, a.z1, a.z2, static_cast<int>(dim), N, j0, nc,
+                              a.incompr ? 1 : 0, range_part, static_cast<int>(rb), maxbits, rec, range_flag));
         tl.end();
-        GSC_CUDA(cudaGetLastError());
         return GSC_OK;
     };
     // the sums of modes [j0, j0 + nc) with records built, into the output

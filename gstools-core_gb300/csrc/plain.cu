@@ -43,6 +43,7 @@
 
 #include "fix64.cuh"
 #include "internal.h"
+#include "launch.cuh"
 
 namespace gsc {
 namespace {
@@ -109,18 +110,15 @@ __device__ __forceinline__ void rec_group(const double *__restrict__ cov, int64_
     for (int i = 0; i < 3; ++i) {
         if (i >= nout) continue;
         int e = -100000;
-        if (regular && a[i] != 0.0) {
-            frexp(a[i], &e);
-            e += ez;
-        }
+        if (regular && a[i] != 0.0) e = exponent_of(a[i]) + ez;
         const int eg = __reduce_max_sync(0xffffffffu, e);
         if (eg == -100000) continue;                             // all zero: scale 0
         if (eg < -900 || eg > 900) {
             regular = false;
             continue;
         }
-        if (regular) fix[i] = __double2ll_rn(ldexp(a[i], ez - eg + 58));
-        scale[i] = ldexp(1.0, eg - 56);
+        if (regular) fix[i] = __double2ll_rn(scale_pow2(a[i], ez - eg + 58));
+        scale[i] = scale_pow2(1.0, eg - 56);
     }
     if (!live) return;
     const Factor f1 = factor_of(k[1]), f2 = factor_of(k[2]);
@@ -151,13 +149,17 @@ __global__ void __launch_bounds__(kThreads)
 plain_rec_kernel(const double *__restrict__ cov, const double *__restrict__ z1,
                  const double *__restrict__ z2, int dim, int64_t n_modes, int64_t j0, int64_t nc,
                  int incompr, double *__restrict__ rec, const int *__restrict__ run_if) {
-    if (run_if && *run_if == 0) return;      // a predicated launch that is not wanted
     __shared__ CosTable tab;
+    if (run_if) {
+        after_previous();
+        if (*run_if == 0) return;            // a predicated launch that is not wanted
+    }
+    fill_cos_table(&tab, threadIdx.x, kThreads);
+    __syncthreads();
+    after_previous();
     const int64_t jl = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x, j = j0 + jl;
     const bool live = jl < nc;
     const double a = live ? z1[j] : 0.0, b = live ? z2[j] : 0.0;
-    fill_cos_table(&tab, threadIdx.x, kThreads);
-    __syncthreads();
     rec_group(cov, n_modes, dim, j, live, a, b, incompr, rec + jl * kRec, &tab);
 }
 
@@ -375,9 +377,13 @@ __global__ void __launch_bounds__(kThreads)
 plain_kernel(const double *__restrict__ pos, int64_t P, const double *__restrict__ rec, int64_t nc,
              int64_t mps, int accumulate, double *__restrict__ dst, int64_t sd, int64_t sp,
              int64_t split_stride, const int *__restrict__ run_if) {
-    if (run_if && *run_if == 0) return;      // a predicated launch that is not wanted
     __shared__ PlainSmem sm;
+    if (run_if) {
+        after_previous();
+        if (*run_if == 0) return;            // a predicated launch that is not wanted
+    }
     if (!LIBM) fill_cos_table(&sm.tab, threadIdx.x, kThreads);   // read after the first tile's barrier
+    after_previous();
     const int64_t jb = static_cast<int64_t>(blockIdx.y) * mps;
     const int64_t je = min(nc, jb + mps);
     plain_block<D, R, INC, LIBM>(pos, P, static_cast<int64_t>(blockIdx.x) * (kThreads * R), rec, jb, je,
@@ -436,6 +442,7 @@ batch_plain_kernel(const BatchItem *__restrict__ items, const BatchUnit *__restr
 __global__ void split_reduce_kernel(const double *__restrict__ part, int64_t S, int64_t nout,
                                     int64_t P, double *__restrict__ out, int64_t sd, int64_t sp,
                                     const int *__restrict__ run_if) {
+    after_previous();
     if (run_if && *run_if == 0) return;      // a predicated launch that is not wanted
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= nout * P) return;
@@ -474,11 +481,17 @@ struct PlainLaunch {
     double *dst;
     int64_t sd, sp, split_stride;
     const int *run_if;
+    bool after;            // overlaps the end of the record kernel
 };
 
 template <int R, bool INC, bool LIBM>
 int dispatch_dim(int64_t dim, dim3 grid, cudaStream_t st, const PlainLaunch &l) {
     auto launch = [&](auto fn) -> int {
+        if (l.after) {
+            GSC_CUDA(launch_after(fn, grid, dim3(kThreads), 0, st, l.pos, l.P, l.rec, l.nc, l.mps, l.accumulate,
+                                  l.dst, l.sd, l.sp, l.split_stride, l.run_if));
+            return GSC_OK;
+        }
         fn<<<grid, kThreads, 0, st>>>(l.pos, l.P, l.rec, l.nc, l.mps, l.accumulate, l.dst, l.sd, l.sp,
                                       l.split_stride, l.run_if);
         GSC_CUDA(cudaGetLastError());
@@ -543,6 +556,19 @@ PlainShape plain_shape(int64_t P, int64_t chunk, int64_t dim, int64_t nout, int 
     return best;
 }
 
+// The shape of a launch that mostly has nothing to do (run_if): few blocks, which
+// each cost time only to look at the word (2,097,152 points x 4096 modes: 137 us
+// of nothing in a real launch's shape, 8 us in 4,096 blocks).
+PlainShape plain_shape_unlikely(int64_t P, int64_t chunk, int sms) {
+    PlainShape s{4, (P + 4 * kThreads - 1) / (4 * kThreads), 1, 0};
+    const int64_t groups = std::max<int64_t>(1, (chunk + kGroup - 1) / kGroup);
+    const int64_t want = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(groups, 64), 4 * sms / s.bx));
+    const int64_t per = (groups + want - 1) / want;
+    s.S = (groups + per - 1) / per;
+    s.mps = per * kGroup;
+    return s;
+}
+
 int sm_count(int device) {
     static std::atomic<int> cached[64];   // zero-initialised (static storage)
     if (device >= 0 && device < 64) {
@@ -590,6 +616,7 @@ __global__ void interleave_kernel(const double *__restrict__ src, int nout, int6
 // summator form compute the Fourier field unchanged.
 __global__ void fourier_scale_kernel(const double *__restrict__ sf, const double *z1,
                                      const double *z2, int64_t n, double *z1s, double *z2s) {
+    after_previous();
     const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const double f = sf[j], a = z1[j], b = z2[j];
@@ -616,10 +643,9 @@ int split_reduce(const double *part, int64_t S, int64_t nout, int64_t P, double 
     TimedLaunch tl(st);
     tl.begin(K_SPLIT_REDUCE);
     const int64_t tot = nout * P;
-    split_reduce_kernel<<<static_cast<unsigned>((tot + 255) / 256), 256, 0, st>>>(part, S, nout, P,
-                                                                                 out, sd, sp, nullptr);
+    GSC_CUDA(launch_after(split_reduce_kernel, dim3(static_cast<unsigned>((tot + 255) / 256)), dim3(256), 0, st,
+                          part, S, nout, P, out, sd, sp, static_cast<const int *>(nullptr)));
     tl.end();
-    GSC_CUDA(cudaGetLastError());
     return GSC_OK;
 }
 
@@ -668,7 +694,8 @@ int plain_run(DeviceCtx &ctx, const PlainArgs &a, cudaStream_t st) {
 
     // ---- launch geometry ---------------------------------------------------
     const int64_t chunk = std::min<int64_t>(N, kChunkModes);
-    const PlainShape shp = plain_shape(P, chunk, dim, nout, sm_count(ctx.device), libm);
+    const PlainShape shp = a.run_if ? plain_shape_unlikely(P, chunk, sm_count(ctx.device))
+                                    : plain_shape(P, chunk, dim, nout, sm_count(ctx.device), libm);
     const int64_t S = shp.S;
     if (shp.bx > 0x7fffffff) return set_error(GSC_ERR_INVALID, "too many points for one launch");
 
@@ -691,6 +718,7 @@ int plain_run(DeviceCtx &ctx, const PlainArgs &a, cudaStream_t st) {
     l.sp = S > 1 ? 1 : a.out_sp;
     l.split_stride = S > 1 ? nout * P : 0;
     l.run_if = a.run_if;
+    l.after = true;
 
     int64_t j0 = 0;
     do {
@@ -698,10 +726,10 @@ int plain_run(DeviceCtx &ctx, const PlainArgs &a, cudaStream_t st) {
         if (nc > 0) {
             TimedLaunch tl(st);
             tl.begin(K_MODE_TABLE);
-            plain_rec_kernel<<<static_cast<unsigned>((nc + kThreads - 1) / kThreads), kThreads, 0, st>>>(
-                a.cov, a.z1, a.z2, static_cast<int>(dim), N, j0, nc, a.incompr ? 1 : 0, rec, a.run_if);
+            GSC_CUDA(launch_after(plain_rec_kernel, dim3(static_cast<unsigned>((nc + kThreads - 1) / kThreads)),
+                                  dim3(kThreads), 0, st, a.cov, a.z1, a.z2, static_cast<int>(dim), N, j0, nc,
+                                  a.incompr ? 1 : 0, rec, a.run_if));
             tl.end();
-            GSC_CUDA(cudaGetLastError());
         }
         l.nc = nc;
         l.mps = shp.mps;
@@ -723,10 +751,9 @@ int plain_run(DeviceCtx &ctx, const PlainArgs &a, cudaStream_t st) {
         TimedLaunch tl(st);
         tl.begin(K_SPLIT_REDUCE);
         const int64_t tot = nout * P;
-        split_reduce_kernel<<<static_cast<unsigned>((tot + 255) / 256), 256, 0, st>>>(
-            part, S, nout, P, a.out, a.out_sd, a.out_sp, a.run_if);
+        GSC_CUDA(launch_after(split_reduce_kernel, dim3(static_cast<unsigned>((tot + 255) / 256)), dim3(256), 0, st,
+                              part, S, nout, P, a.out, a.out_sd, a.out_sp, a.run_if));
         tl.end();
-        GSC_CUDA(cudaGetLastError());
     }
     GSC_CUDA(cudaEventRecord(ctx.scratch_ready, st));
     return GSC_OK;

@@ -24,6 +24,7 @@
 #include <algorithm>
 
 #include "internal.h"
+#include "launch.cuh"
 
 namespace gsc {
 namespace {
@@ -95,6 +96,7 @@ __device__ void f64_gtab_entry(const F64Tab &t, int64_t i) {
 
 // s, B and G tables: a fixed grid strides over all entries
 __global__ void __launch_bounds__(256) f64_tables_kernel(F64Tab t) {
+    after_previous();
     if (t.run_if && *t.run_if == 0) return;
     const int64_t n1 = static_cast<int64_t>(t.nb) * t.n_modes, n2 = static_cast<int64_t>(t.n_modes) * t.nm;
     const int64_t n3 = static_cast<int64_t>(t.ncn_pad) * (t.k_pad / 2);
@@ -125,6 +127,7 @@ struct F64Params {
 
 __global__ void __launch_bounds__(kF64Threads)
 sep_f64_kernel(const F64Params p) {
+    after_previous();
     if (p.run_if && *p.run_if == 0) return;
     __shared__ double As[TM * LDS];
     __shared__ double Bs[TN * LDS];
@@ -278,15 +281,14 @@ int sep_f64_launch(const SepArgs &a, unsigned char *base, const int *run_if, cud
     {
         TimedLaunch tl(st);
         tl.begin(K_SEP_TABLES);
-        f64_tables_kernel<<<kF64Grid, 256, 0, st>>>(t);
+        GSC_CUDA(launch_after(f64_tables_kernel, dim3(kF64Grid), dim3(256), 0, st, t));
         tl.end();
-        GSC_CUDA(cudaGetLastError());
     }
     TimedLaunch tl(st);
     tl.begin(K_SEP_F64);
-    sep_f64_kernel<<<static_cast<unsigned>(std::min<int64_t>(p.tiles, kF64Grid)), kF64Threads, 0, st>>>(p);
+    GSC_CUDA(launch_after(sep_f64_kernel, dim3(static_cast<unsigned>(std::min<int64_t>(p.tiles, kF64Grid))),
+                          dim3(kF64Threads), 0, st, p));
     tl.end();
-    GSC_CUDA(cudaGetLastError());
     return GSC_OK;
 }
 

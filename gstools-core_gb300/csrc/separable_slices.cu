@@ -52,6 +52,7 @@
 
 #include "fix64.cuh"
 #include "internal.h"
+#include "launch.cuh"
 #include "sm100.cuh"
 
 namespace gsc {
@@ -103,12 +104,19 @@ struct SlTab {
     int *words;
 };
 
+// the least e with |x| <= 2^e, x != 0
+__device__ __forceinline__ int ceil_exponent(double x) {
+    const int e = exponent_of(x);
+    return e - (fabs(x) == scale_pow2(0.5, e) ? 1 : 0);
+}
+
 // z1 + i z2 of every mode as amplitude and angle, projector weights and the
 // exponents of the largest.
 __global__ void __launch_bounds__(128) sl_modes_kernel(SlTab t) {
     __shared__ CosTable tab;
     fill_cos_table(&tab, threadIdx.x, 128);
     __syncthreads();
+    after_previous();
     const int j = blockIdx.x * 128 + threadIdx.x;
     const bool live = j < t.n_modes;
     int top[4] = {0, 0, 0, 0};
@@ -136,18 +144,12 @@ __global__ void __launch_bounds__(128) sl_modes_kernel(SlTab t) {
         if (!bad) {
             mode_angle(z1, z2, &tab, &m.amp, &m.ez, &m.beta);
             if (m.amp > 0.0) {
-                int e;
-                const double f = frexp(m.amp, &e);
-                m.ea = m.ez + e - (f == 0.5 ? 1 : 0);          // A <= 2^ea
+                m.ea = m.ez + ceil_exponent(m.amp);            // A <= 2^ea
                 bad = m.ea < -900 || m.ea > 900;
                 top[0] = m.ea + kWordBias;
             }
             for (int c = 0; c < t.ncomp; ++c)
-                if (m.w[c] != 0.0) {
-                    int e;
-                    const double f = frexp(fabs(m.w[c]), &e);
-                    top[1 + c] = e - (f == 0.5 ? 1 : 0) + kWordBias;   // |w| <= 2^e
-                }
+                if (m.w[c] != 0.0) top[1 + c] = ceil_exponent(m.w[c]) + kWordBias;   // |w| <= 2^e
         }
         t.modes[j] = m;
     }
@@ -202,6 +204,7 @@ sl_tables_kernel(SlTab t, int64_t n_g, int64_t n_b, int64_t n_s) {
     __shared__ CosTable tab;
     fill_cos_table(&tab, threadIdx.x, kTabThreads);
     __syncthreads();
+    after_previous();
     const int np = t.kb * kKbModes;
     const int ew = top_exponent(t.words[1]);
     bool bad = false;
@@ -231,7 +234,7 @@ sl_tables_kernel(SlTab t, int64_t n_g, int64_t n_b, int64_t n_s) {
                     int64_t co, si;
                     cis_fine(fraction(t.dim - 1, j, t.ax_n[n]) + kFineOffset, &tab, &co, &si);
                     const int g = t.incompr ? top_exponent(t.words[2 + comp]) : 0;
-                    const int64_t wf = __double2ll_rn(ldexp(m.w[comp], 62 - g - mode_shift(m, ew)));
+                    const int64_t wf = __double2ll_rn(scale_pow2(m.w[comp], 62 - g - mode_shift(m, ew)));
                     re = __mul64hi(wf, co);
                     im = -__mul64hi(wf, si);
                 }
@@ -267,7 +270,7 @@ sl_tables_kernel(SlTab t, int64_t n_g, int64_t n_b, int64_t n_s) {
                 if (t.dim == 3) th += fraction(0, j, t.ax_b[b]);
                 int64_t co, si;
                 cis_fine(th, &tab, &co, &si);
-                const int64_t a = __double2ll_rn(ldexp(m.amp, m.ez - ew + mode_shift(m, ew) + 62));
+                const int64_t a = __double2ll_rn(scale_pow2(m.amp, m.ez - ew + mode_shift(m, ew) + 62));
                 v = make_longlong2(__mul64hi(a, co) << 2, __mul64hi(a, si) << 2);
             }
             t.svec[i] = v;
@@ -299,6 +302,7 @@ __device__ __forceinline__ int64_t dot_fixed(Word2 a, Word2 b, Word2 c, Word2 d)
 // thread, which share s, 139).
 constexpr int kSliceThreads = 256;
 __global__ void __launch_bounds__(kSliceThreads, 5) sl_slice_kernel(SlTab t) {
+    after_previous();
     if (t.words[0]) return;
     const int c = threadIdx.x & 3, r = (blockIdx.x & 1) * 64 + (threadIdx.x >> 2);
     const int kb = blockIdx.y;
@@ -440,6 +444,7 @@ __device__ __forceinline__ double scaled_total(int64_t t, int e) {
 template <int NT>
 __global__ void __launch_bounds__(kThreads, 1) sl_gemm_kernel(const SlGemm p) {
     using L = SlLayout<NT>;
+    after_previous();
     if (p.words[0]) return;          // the same for every CTA
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>(
@@ -729,6 +734,7 @@ __global__ void __launch_bounds__(kThreads, 1) sl_gemm_kernel(const SlGemm p) {
 __global__ void __launch_bounds__(256)
 sl_reduce_kernel(const int64_t *__restrict__ part, int segs, int splits, int last, int64_t P, int ncomp,
                  int finer, double *__restrict__ out, const int *__restrict__ words) {
+    after_previous();
     if (words[0]) return;
     const int64_t q = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x, n = ncomp * P;
     if (q >= P) return;
@@ -750,8 +756,8 @@ sl_reduce_kernel(const int64_t *__restrict__ part, int segs, int splits, int las
 template <int NT>
 int launch_gemm(const SlGemm &p, int64_t grid, cudaStream_t st) {
     GSC_TRY(smem_attr(reinterpret_cast<const void *>(sl_gemm_kernel<NT>), SlLayout<NT>::SMEM));
-    sl_gemm_kernel<NT><<<static_cast<unsigned>(grid), kThreads, SlLayout<NT>::SMEM, st>>>(p);
-    GSC_CUDA(cudaGetLastError());
+    GSC_CUDA(launch_after(sl_gemm_kernel<NT>, dim3(static_cast<unsigned>(grid)), dim3(kThreads),
+                          SlLayout<NT>::SMEM, st, p));
     return GSC_OK;
 }
 
@@ -906,9 +912,9 @@ int sep_slices_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
             const int64_t blocks = (n_g + kTabThreads - 1) / kTabThreads + (n_b + kTabThreads - 1) / kTabThreads +
                                    (n_s + kTabThreads - 1) / kTabThreads;
             if (blocks > 0x7fffffff) return set_error(GSC_ERR_INVALID, "tables too large");
-            sl_tables_kernel<<<static_cast<unsigned>(blocks), kTabThreads, 0, st>>>(t, n_g, n_b, n_s);
+            GSC_CUDA(launch_after(sl_tables_kernel, dim3(static_cast<unsigned>(blocks)), dim3(kTabThreads), 0, st,
+                                  t, n_g, n_b, n_s));
             tl.end();
-            GSC_CUDA(cudaGetLastError());
         }
         for (int64_t m0 = 0; m0 < pl.m_tiles; m0 += pl.slab) {
             const int64_t mts = std::min(pl.slab, pl.m_tiles - m0);
@@ -916,10 +922,9 @@ int sep_slices_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
             {
                 TimedLaunch tl(st);
                 tl.begin(K_SEP_SPLIT);
-                sl_slice_kernel<<<dim3(static_cast<unsigned>(2 * mts), static_cast<unsigned>(t.kb)),
-                                  kSliceThreads, 0, st>>>(t);
+                GSC_CUDA(launch_after(sl_slice_kernel, dim3(static_cast<unsigned>(2 * mts), static_cast<unsigned>(t.kb)),
+                                      dim3(kSliceThreads), 0, st, t));
                 tl.end();
-                GSC_CUDA(cudaGetLastError());
             }
             SlGemm p{};
             p.f = t.f;
@@ -958,10 +963,10 @@ int sep_slices_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
         const int kb_last = (N - (pl.segs - 1) * kSegModes + kKbModes - 1) / kKbModes;
         TimedLaunch tl(st);
         tl.begin(K_SPLIT_REDUCE);
-        sl_reduce_kernel<<<dim3(static_cast<unsigned>((P + 255) / 256), ncomp), 256, 0, st>>>(
-            part, pl.segs, pl.splits, std::min(pl.splits, kb_last), P, ncomp, finer, a.out, t.words);
+        GSC_CUDA(launch_after(sl_reduce_kernel, dim3(static_cast<unsigned>((P + 255) / 256), ncomp), dim3(256), 0, st,
+                              part, pl.segs, pl.splits, std::min(pl.splits, kb_last), P, ncomp, finer, a.out,
+                              t.words));
         tl.end();
-        GSC_CUDA(cudaGetLastError());
     }
     // inputs outside this form: the FP64 MMA kernels, which do nothing otherwise
     GSC_TRY(sep_f64_launch(a, base + 256, t.words, st));

@@ -50,6 +50,7 @@
 
 #include "dfturns.cuh"
 #include "internal.h"
+#include "launch.cuh"
 #include "sm100.cuh"
 
 namespace gsc {
@@ -669,6 +670,7 @@ __device__ void wnorm_block(const double *__restrict__ z1, const double *__restr
 constexpr int kRecX5 = 16;   // kh0-2 kl0-2 z1h z2h z1l z2l wh0-2 wl0-2
 
 __global__ void __launch_bounds__(256) sep_x5_split_kernel(TabArgs t, int64_t n_ax) {
+    after_previous();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < t.n_modes) {
         const int j = static_cast<int>(i);
@@ -851,6 +853,7 @@ __device__ __forceinline__ void gtab_x5_entry(const TabArgs &t, int64_t i) {
 // B-table elements.
 __global__ void __launch_bounds__(256)
 sep_x5_tables_kernel(TabArgs t, int64_t n_svec, int64_t n_btab, int64_t n_gtab) {
+    after_previous();
     if (blockIdx.x == 0) {
         wnorm_block(t.z1, t.z2, t.n_modes, t.kbt, t.kc, t.wnorm, t.l1kb, t.bound_flag, t.bound_sticky);
         return;
@@ -975,6 +978,7 @@ __global__ void __launch_bounds__(X5_THREADS, 1)
 sep_x5_kernel(const __grid_constant__ CUtensorMap out_map, const X5Params xp) {
     using L = X5Layout<BNX>;
     const TcParams &p = xp.base;
+    after_previous();
     // inputs whose main sum could leave FP32's exact range are not computed
     // (the flag is the same for every CTA, so whole CTAs leave before any
     // barrier or TMEM allocation)
@@ -1772,7 +1776,7 @@ int sep_tc_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
             sep_x5_split_kernel<<<static_cast<unsigned>((ns + 255) / 256), 256, 0, st>>>(t, n_ax);
             tl.end();
             tl.begin(K_SEP_TABLES);
-            sep_x5_tables_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(t, n1, n2, ng);
+            GSC_CUDA(launch_after(sep_x5_tables_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, t, n1, n2, ng));
             tl.end();
         } else {
             if (n1 > 0) {
@@ -1876,16 +1880,16 @@ int sep_tc_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
             const unsigned g = static_cast<unsigned>(l.full_tiles + l.n_split * l.ksplit);
             if (bnx == 192 && l.n_split > 0) {
                 GSC_TRY((configure_x5<192, true>()));
-                sep_x5_kernel<192, true><<<g, X5_THREADS, X5Layout<192>::SMEM, st>>>(om, xp);
+                GSC_CUDA(launch_after(sep_x5_kernel<192, true>, dim3(g), dim3(X5_THREADS), X5Layout<192>::SMEM, st, om, xp));
             } else if (bnx == 192) {
                 GSC_TRY((configure_x5<192, false>()));
-                sep_x5_kernel<192, false><<<g, X5_THREADS, X5Layout<192>::SMEM, st>>>(om, xp);
+                GSC_CUDA(launch_after(sep_x5_kernel<192, false>, dim3(g), dim3(X5_THREADS), X5Layout<192>::SMEM, st, om, xp));
             } else if (l.n_split > 0) {
                 GSC_TRY((configure_x5<256, true>()));
-                sep_x5_kernel<256, true><<<g, X5_THREADS, X5Layout<256>::SMEM, st>>>(om, xp);
+                GSC_CUDA(launch_after(sep_x5_kernel<256, true>, dim3(g), dim3(X5_THREADS), X5Layout<256>::SMEM, st, om, xp));
             } else {
                 GSC_TRY((configure_x5<256, false>()));
-                sep_x5_kernel<256, false><<<g, X5_THREADS, X5Layout<256>::SMEM, st>>>(om, xp);
+                GSC_CUDA(launch_after(sep_x5_kernel<256, false>, dim3(g), dim3(X5_THREADS), X5Layout<256>::SMEM, st, om, xp));
             }
             GSC_CUDA(cudaGetLastError());
             if (a.on_rows)
