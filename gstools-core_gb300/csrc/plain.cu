@@ -236,6 +236,7 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
     // read from pos where they are needed)
     double x0[R];
     Factor xf[R][D > 1 ? D - 1 : 1];
+    double x1[R];                            // D == 2: the second coordinate of odd r
     double acc[R][NOUT];
     double xabs = 0.0;
     bool bad[R];
@@ -253,6 +254,7 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
                 x0[r] = x;
             } else {
                 xf[r][d - 1] = factor_of(x);
+                x1[r] = x;
                 if (!factor_in_range(x) && !isnan(x)) xabs = __longlong_as_double(0x7ff0000000000000ll);
             }
         }
@@ -297,6 +299,7 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
                                       {static_cast<uint32_t>(__double2loint(q1.x)), static_cast<uint32_t>(__double2hiint(q1.x)),
                                        static_cast<uint32_t>(__double2hiint(q1.y))}};
                 const uint64_t beta = static_cast<uint64_t>(__double_as_longlong(q2.x));
+                const double k1 = kf[0].value();
                 double av[3] = {q2.y, 0.0, 0.0};
                 if (INC) {
                     const double2 q3 = mr[3];
@@ -308,7 +311,10 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
                     // as phase_of
                     double ph = __dmul_rn(q0.x, x0[r]);
 #pragma unroll
-                    for (int d = 1; d < D; ++d) ph = __dadd_rn(ph, rn_product(kf[d - 1], xf[r][d - 1]));
+                    for (int d = 1; d < D; ++d) {
+                        const bool fp64 = D == 2 && (r & 1);
+                        ph = __dadd_rn(ph, fp64 ? __dmul_rn(k1, x1[r]) : rn_product(kf[d - 1], xf[r][d - 1]));
+                    }
                     const int64_t c = cos_fixed(turn_fraction(ph) + beta, &sm.tab);
                     const int32_t ch = static_cast<int32_t>(c >> 32);
                     const int32_t c0 = static_cast<int32_t>(static_cast<uint32_t>(c) >> 1);
