@@ -274,14 +274,6 @@ fx_mode_kernel(const double *__restrict__ cov, const double *__restrict__ z1,
     fx_mode_entry(k, z1j, z2j, dim, incompr, mb, maxbits + 3, rec + jl * kFxRecWords, range_flag);
 }
 
-// Kahan step: (sum, cmp) += a, cmp holding minus the lost low-order part
-__device__ __forceinline__ void fx_kahan(float &sum, float &cmp, float a) {
-    const float y = a - cmp;
-    const float t = sum + y;
-    cmp = (t - sum) - y;
-    sum = t;
-}
-
 // Knuth's TwoSum: (hi, lo) += a
 __device__ __forceinline__ void fx_two_sum(float &hi, float &lo, float a) {
     const float s = hi + a;
@@ -298,38 +290,87 @@ __device__ __forceinline__ float2 fx_lds2(uint32_t addr) {
     return v;
 }
 
-// The term Re(T e^{i theta}) of one point*mode: c the point's constant,
-// (xh, x8l / xlf) its coordinate words, (bi, bf / bif) the mode's
+// Two FP32 values in a register pair, and operations on both (each as the FP32
+// instruction rounds it, in half the issue slots).
+struct F2 {
+    uint64_t v;
+    __device__ __forceinline__ float lo() const { return __uint_as_float(static_cast<uint32_t>(v)); }
+    __device__ __forceinline__ float hi() const { return __uint_as_float(static_cast<uint32_t>(v >> 32)); }
+};
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ F2 f2(float x) { return f2(x, x); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
+// Kahan steps of two points: (sum, cmp) += a, cmp holding minus the lost
+// low-order part
+__device__ __forceinline__ void fx_kahan2(F2 &sum, F2 &cmp, F2 a) {
+    const F2 y = sub2(a, cmp);
+    const F2 t = add2(sum, y);
+    cmp = sub2(sub2(t, sum), y);
+    sum = t;
+}
+
+// The terms Re(T e^{i theta}) of a mode at two points: c the points' constants,
+// (xh, x8l / xlf) their coordinate words, (bi, bf / bif) the mode's
 // wave-number words, tab the shared-memory address of the mode's
 // 128-byte-aligned table.
 template <int D, bool SMALL>
-__device__ __forceinline__ float fx_term(uint32_t c, const uint32_t *xh, const uint32_t *x8l,
-                                         const float *xlf, const uint32_t *bi, const uint32_t *bf,
-                                         const float *bif, uint32_t tab) {
-    uint32_t t = c;
+__device__ __forceinline__ F2 fx_term(const uint32_t *c, const uint32_t (*xh)[D], const uint32_t (*x8l)[SMALL ? 1 : D],
+                                      const F2 *xlf, const uint32_t *bi, const uint32_t *bf,
+                                      const float *bif, uint32_t tab) {
+    uint32_t t[2] = {c[0], c[1]};
     if constexpr (SMALL) {
         // sum_d BI Xl 2^-29 (every |BI| < 2^20) rounded to an integer by a
         // chain of FP32 fused multiply-adds into the mantissa of 1.5 2^23
-        float v = kFxMagic;
+        F2 v = f2(kFxMagic);
 #pragma unroll
-        for (int d = 0; d < D; ++d) v = fmaf(bif[d], xlf[d], v);
-        t += __float_as_uint(v);
+        for (int d = 0; d < D; ++d) v = fma2(f2(bif[d]), xlf[d], v);
+        t[0] += __float_as_uint(v.lo());
+        t[1] += __float_as_uint(v.hi());
     }
+    float2 T[2];
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-        if constexpr (!SMALL) t += __umulhi(bi[d], x8l[d]);
-        t += __umulhi(bf[d], xh[d]);
-        t += bi[d] * xh[d];
+    for (int q = 0; q < 2; ++q) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            if constexpr (!SMALL) t[q] += __umulhi(bi[d], x8l[q][d]);
+            t[q] += __umulhi(bf[d], xh[q][d]);
+            t[q] += bi[d] * xh[q][d];
+        }
+        // t = theta + 2^27 + 16: entry m = t >> 28 (theta to the nearest 1/16
+        // turn) at byte 8 m of the table; bits 5..27 are the remainder plus
+        // 1/32 turn in units of 2^-27 turn, as the mantissa of a float in [1, 2)
+        T[q] = fx_lds2(tab | ((t[q] >> 25) & 0x78u));
+        t[q] = 0x3F800000u | ((t[q] >> 5) & 0x007FFFFFu);
     }
-    // t = theta + 2^27 + 16: entry m = t >> 28 (theta to the nearest 1/16
-    // turn) at byte 8 m of the table; bits 5..27 are the remainder plus
-    // 1/32 turn in units of 2^-27 turn, as the mantissa of a float in [1, 2)
-    const float2 T = fx_lds2(tab | ((t >> 25) & 0x78u));
-    const float r = __uint_as_float(0x3F800000u | ((t >> 5) & 0x007FFFFFu)) - 1.5f;
-    const float r2 = r * r;
-    const float sn = r * fmaf(r2, fmaf(r2, kFxS5, kFxS3), kFxS1);
-    const float cs = fmaf(r2, fmaf(r2, kFxC4, kFxC2), kFxC0);
-    return fmaf(T.x, cs, -T.y * sn);
+    const F2 r = add2(f2(__uint_as_float(t[0]), __uint_as_float(t[1])), f2(-1.5f));
+    const F2 r2 = mul2(r, r);
+    const F2 sn = mul2(r, fma2(r2, fma2(r2, f2(kFxS5), f2(kFxS3)), f2(kFxS1)));
+    const F2 cs = fma2(r2, fma2(r2, f2(kFxC4), f2(kFxC2)), f2(kFxC0));
+    return f2(fmaf(T[0].x, cs.lo(), -T[0].y * sn.lo()), fmaf(T[1].x, cs.hi(), -T[1].y * sn.hi()));
 }
 
 // The words of mode m of the staged tile: BI' and BF, BI as FP32, the
@@ -384,7 +425,7 @@ __device__ __forceinline__ void fx_block_(const double *__restrict__ pos, int64_
     // SMALL: every mode's |BI| < 2^20, and BI Xl 2^-29 is an FP32 product
     // (xlf = Xl 2^-29); otherwise a high integer product (x8l = 8 Xl)
     uint32_t xh[R][D], x8l[R][SMALL ? 1 : D], cp[R];
-    float xlf[R][SMALL ? D : 1];
+    F2 xlf[R / 2][SMALL ? D : 1];
     bool bad[R];
     float hi[R][NOUT], lo[R][NOUT];
 #pragma unroll
@@ -405,7 +446,8 @@ __device__ __forceinline__ void fx_block_(const double *__restrict__ pos, int64_
             const uint32_t l = static_cast<uint32_t>(Xp) & 0x1FFFFFFFu;
             xh[r][d] = h;
             if constexpr (SMALL) {
-                xlf[r][d] = static_cast<float>(l) * 1.862645149230957e-09f;     // Xl 2^-29
+                const float f = static_cast<float>(l) * 1.862645149230957e-09f;     // Xl 2^-29
+                xlf[r / 2][d] = (r & 1) ? f2(xlf[r / 2][d].lo(), f) : f2(f);
                 // the bias 2^31 of BI' adds 2^31 Xh (mod 2^32)
                 c -= (h & 1u) << 31;
             } else {
@@ -435,37 +477,37 @@ __device__ __forceinline__ void fx_block_(const double *__restrict__ pos, int64_
             }
         }
         __syncthreads();
-        float acc[R][NOUT], cmp[R][NOUT];
+        F2 acc[R / 2][NOUT], cmp[R / 2][NOUT];
 #pragma unroll
-        for (int r = 0; r < R; ++r)
+        for (int r = 0; r < R / 2; ++r)
 #pragma unroll
-            for (int i = 0; i < NOUT; ++i) acc[r][i] = cmp[r][i] = 0.f;
+            for (int i = 0; i < NOUT; ++i) acc[r][i] = cmp[r][i] = f2(0.f);
         // modes in groups of eight: four pair sums per point, added, then one
         // Kahan step; a tile shorter than TILE (the last) goes in pairs,
         // the second mode of an odd tile's last pair counting zero times
         constexpr int kGroupPairs = 4;
         const int tq = tm == TILE ? TILE : 0;
         for (int m = 0; m < tq; m += 2 * kGroupPairs) {
-            float pend[R][NOUT];
+            F2 pend[R / 2][NOUT];
 #pragma unroll
             for (int h = 0; h < kGroupPairs; ++h) {
                 const FxModeWords ma = fx_mode_words<INC>(srec, sbase, m + 2 * h, 1.0f);
                 const FxModeWords mb = fx_mode_words<INC>(srec, sbase, m + 2 * h + 1, 1.0f);
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const float ta = fx_term<D, SMALL>(cp[r], xh[r], x8l[r], xlf[r], ma.bi,
-                                                       ma.bf, ma.bif, ma.tab);
-                    const float tb = fx_term<D, SMALL>(cp[r], xh[r], x8l[r], xlf[r], mb.bi,
-                                                       mb.bf, mb.bif, mb.tab);
+                for (int r = 0; r < R / 2; ++r) {
+                    const F2 ta = fx_term<D, SMALL>(&cp[2 * r], &xh[2 * r], &x8l[2 * r], xlf[r], ma.bi,
+                                                    ma.bf, ma.bif, ma.tab);
+                    const F2 tb = fx_term<D, SMALL>(&cp[2 * r], &xh[2 * r], &x8l[2 * r], xlf[r], mb.bi,
+                                                    mb.bf, mb.bif, mb.tab);
 #pragma unroll
                     for (int i = 0; i < NOUT; ++i) {
-                        const float ps = INC ? fmaf(ma.w[i], ta, mb.w[i] * tb) : ta + tb;
+                        const F2 ps = INC ? fma2(f2(ma.w[i]), ta, mul2(f2(mb.w[i]), tb)) : add2(ta, tb);
                         if (h == 0)
                             pend[r][i] = ps;
                         else if (h < kGroupPairs - 1)
-                            pend[r][i] += ps;
+                            pend[r][i] = add2(pend[r][i], ps);
                         else
-                            fx_kahan(acc[r][i], cmp[r][i], pend[r][i] + ps);
+                            fx_kahan2(acc[r][i], cmp[r][i], add2(pend[r][i], ps));
                     }
                 }
             }
@@ -476,23 +518,24 @@ __device__ __forceinline__ void fx_block_(const double *__restrict__ pos, int64_
             const FxModeWords ma = fx_mode_words<INC>(srec, sbase, m, 1.0f);
             const FxModeWords mb = fx_mode_words<INC>(srec, sbase, two ? m + 1 : m, sb);
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const float ta = fx_term<D, SMALL>(cp[r], xh[r], x8l[r], xlf[r], ma.bi, ma.bf,
-                                                   ma.bif, ma.tab);
-                const float tb = fx_term<D, SMALL>(cp[r], xh[r], x8l[r], xlf[r], mb.bi, mb.bf,
-                                                   mb.bif, mb.tab);
+            for (int r = 0; r < R / 2; ++r) {
+                const F2 ta = fx_term<D, SMALL>(&cp[2 * r], &xh[2 * r], &x8l[2 * r], xlf[r], ma.bi, ma.bf,
+                                                ma.bif, ma.tab);
+                const F2 tb = fx_term<D, SMALL>(&cp[2 * r], &xh[2 * r], &x8l[2 * r], xlf[r], mb.bi, mb.bf,
+                                                mb.bif, mb.tab);
 #pragma unroll
                 for (int i = 0; i < NOUT; ++i)
-                    fx_kahan(acc[r][i], cmp[r][i],
-                             INC ? fmaf(ma.w[i], ta, mb.w[i] * tb) : fmaf(sb, tb, ta));
+                    fx_kahan2(acc[r][i], cmp[r][i],
+                              INC ? fma2(f2(ma.w[i]), ta, mul2(f2(mb.w[i]), tb)) : fma2(f2(sb), tb, ta));
             }
         }
 #pragma unroll
         for (int r = 0; r < R; ++r)
 #pragma unroll
             for (int i = 0; i < NOUT; ++i) {
-                fx_two_sum(hi[r][i], lo[r][i], acc[r][i]);
-                lo[r][i] -= cmp[r][i];
+                const F2 s = acc[r / 2][i], c = cmp[r / 2][i];
+                fx_two_sum(hi[r][i], lo[r][i], (r & 1) ? s.hi() : s.lo());
+                lo[r][i] -= (r & 1) ? c.hi() : c.lo();
             }
     }
 
