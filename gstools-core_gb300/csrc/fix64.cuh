@@ -177,11 +177,8 @@ constexpr uint64_t kFine2 = 0x34a34cc4a60fa646ull;     // f2 2^76
 constexpr uint64_t kFine3 = 0x000022a264558fb1ull;     // f3 2^75
 constexpr uint64_t kFine4 = 0x34a34cc4a60fa646ull;     // f4 2^75
 constexpr uint64_t kFine5 = 0x000033f396805789ull;     // f5 2^74
-__device__ __forceinline__ void cis_fine(uint64_t theta, const CosTable *tab, int64_t *cosine, int64_t *sine) {
-    const uint32_t a = static_cast<uint32_t>(theta >> 56);
-    const uint4 e = tab->wide[a], g = tab->wide[(a + 192) & 255];
-    const int64_t c = static_cast<int64_t>((static_cast<uint64_t>(e.y) << 32) | e.x);
-    const int64_t s = static_cast<int64_t>((static_cast<uint64_t>(g.y) << 32) | g.x);
+// (c, s: cos and sin of the table step theta >> 56)
+__device__ __forceinline__ void cis_from(uint64_t theta, int64_t c, int64_t s, int64_t *cosine, int64_t *sine) {
     // rho 2^64 and rho^2 2^65 (at most 2^63)
     const int64_t rho = static_cast<int64_t>((theta << 8) ^ (uint64_t(1) << 63));
     const uint64_t q = static_cast<uint64_t>(__mul64hi(rho, rho)) << 1;
@@ -195,6 +192,19 @@ __device__ __forceinline__ void cis_fine(uint64_t theta, const CosTable *tab, in
     const int64_t sn = __mul64hi(rs, static_cast<int64_t>(kStep69 >> 1));
     *cosine = c - (((__mul64hi(c, ver) >> 8) + __mul64hi(s, sn) + 8) >> 4);
     *sine = s - (((__mul64hi(s, ver) >> 8) - __mul64hi(c, sn) + 8) >> 4);
+}
+__device__ __forceinline__ void cis_fine(uint64_t theta, const CosTable *tab, int64_t *cosine, int64_t *sine) {
+    const uint32_t a = static_cast<uint32_t>(theta >> 56);
+    const uint4 e = tab->wide[a], g = tab->wide[(a + 192) & 255];
+    const int64_t c = static_cast<int64_t>((static_cast<uint64_t>(e.y) << 32) | e.x);
+    const int64_t s = static_cast<int64_t>((static_cast<uint64_t>(g.y) << 32) | g.x);
+    cis_from(theta, c, s, cosine, sine);
+}
+// The same without a table in shared memory: for one value per thread, two
+// reads of the quarter wave cost less than the table's set-up.
+__device__ __forceinline__ void cis_fine(uint64_t theta, int64_t *cosine, int64_t *sine) {
+    const int a = static_cast<int>(theta >> 56);
+    cis_from(theta, quarter_cos(a), quarter_cos(a - 64), cosine, sine);
 }
 
 // An FP64 factor for rn_product: the mantissa left-aligned in 64 bits, and the

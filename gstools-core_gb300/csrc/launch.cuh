@@ -18,6 +18,13 @@ __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
 }
 
+// after_previous in two steps, for a kernel of few blocks before one that fills
+// the GPU: wait_previous, then next_may_start at the end.  Blocks of the next
+// kernel that came earlier would find SMs partly taken, and run as a wave of
+// their own.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <class... P, class... A>
 inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                 A... args) {

@@ -25,7 +25,7 @@
 //    FP32 rate);
 //  * e^{i theta}: theta + 2^27 + 16 selects by its top 4 bits one of 16
 //    entries of the mode's table T[m] = (z1 - i z2) e^{2 pi i (m/16 - phi)}
-//    (phi the per-mode constant; built in FP64 per mode, stored as FP32).
+//    (phi the per-mode constant; built to FP64 precision per mode, stored as FP32).
 //    Bits 5..27 of the same word, placed under the exponent of 1.0f, give
 //    1 + u 2^-23 exactly; minus 1.5 that is the remainder r in sixteenths
 //    of a turn (|r| <= 1/2, rounded to 2^-27 turn by the + 16) with no
@@ -46,6 +46,7 @@
 #include <algorithm>
 
 #include "dfturns.cuh"
+#include "fix64.cuh"
 #include "internal.h"
 #include "launch.cuh"
 
@@ -83,14 +84,6 @@ constexpr uint32_t kFxMagicBits = 0x4B400000u;
 // the FP32 product form needs |BI| < 2^20 in every dimension (the sum of
 // three products stays within 2^22 of the magic constant)
 constexpr int32_t kFxSmallBI = 1 << 20;
-
-// cos(2 pi m / 16), m = 0..15, to FP64 rounding (from cos(pi/8) =
-// sqrt(2 + sqrt 2) / 2 and cos(pi/4) = sqrt(2) / 2)
-__constant__ double kSixteenthCos[16] = {
-    1.0, 0.9238795325112867, 0.7071067811865476, 0.38268343236508984,
-    0.0, -0.38268343236508984, -0.7071067811865476, -0.9238795325112867,
-    -1.0, -0.9238795325112867, -0.7071067811865476, -0.38268343236508984,
-    0.0, 0.38268343236508984, 0.7071067811865476, 0.9238795325112867};
 
 // Fixed-point scale s_d of dimension d from the largest finite |x_d|
 // (bits of that non-negative double, 0 when none): |x| * 2^s < 2^60.
@@ -170,108 +163,119 @@ fx_range_kernel(const double *__restrict__ pos, int64_t P, int dim,
     if (blockIdx.x == 0 && threadIdx.x == 0) maxbits[3] = 0ull;
 }
 
-// The record of mode j (see kFxRecWords).  mb[d]: the range words of the
-// positions (largest |x_d| as bits); small_word: set when a wave number
-// needs the general product form.  range_flag (may be null) is set to 1
-// when a wave number is too large for the integer phase at these positions.
-__device__ void fx_mode_entry(const double *k, double z1, double z2, int dim, int incompr,
-                              const unsigned long long *mb, unsigned long long *small_word,
-                              uint32_t *__restrict__ r, int *range_flag) {
-    bool finite = isfinite(z1) && isfinite(z2);
-    bool small = true;                              // every |BI| < 2^20
-    double phi = 0.0;                               // units of 2^-32 turn
-    for (int d = 0; d < 3; ++d) {
-        int32_t bi = 0;
-        uint32_t bf = 0;
-        if (d < dim) {
-            finite = finite && isfinite(k[d]);
-            const double B = fx_ldexp(k[d] * kInv2Pi, 61 - fx_scale(mb[d]));
-            if (fabs(B) < 2147483648.0) {
-                const long long bq = __double2ll_rn(B * 4294967296.0);  // B to 2^-32 (exact scaling)
-                bi = static_cast<int32_t>(bq >> 32);
-                bf = static_cast<uint32_t>(bq);
-                // B 2^31 mod 2^32: what the offset 2^60 of X adds to theta
-                phi += static_cast<double>(static_cast<uint32_t>(bq >> 1)) + 0.5 * (bq & 1);
-            } else if (isfinite(B) && range_flag) {
-                *range_flag = 1;
-            }
+// Records (see kFxRecWords), four neighbouring lanes per mode; all lanes of a
+// warp call, live: the lane's mode exists.  Lane l holds the wave number of
+// dimension l (0 beyond dim) and makes its words, then the table's entries l, l + 4,
+// l + 8 and l + 12, quarter turns of one rotation.  mb[d]: the range words of the
+// positions (largest |x_d| as bits); small_word: set when a wave number needs
+// the general product form.  range_flag (may be null) is set to 1 when a wave
+// number is too large for the integer phase at these positions.
+//
+// A mode is one chain of dependent operations, whose latency every small call
+// waits for: one thread per mode with CUDA's sincos() and 64 FP64 products took
+// 13 us; the rotation of the per-mode constant is exact in 64-bit fixed point
+// here (its cosine within 1e-17), and a lane has four FP64 products.
+__device__ __forceinline__ void fx_mode_entry(bool live, double k, double z1, double z2, int dim, int incompr,
+                                              const unsigned long long *mb, unsigned long long *small_word,
+                                              uint32_t *__restrict__ r, int *range_flag) {
+    const int lane = threadIdx.x & 31, l = lane & 3, g0 = lane & ~3;
+    int32_t bi = 0;
+    uint32_t bf = 0;
+    long long bq = 0;
+    bool flag = false;
+    if (l < dim) {
+        const double B = fx_ldexp(k * kInv2Pi, 61 - fx_scale(l == 0 ? mb[0] : l == 1 ? mb[1] : mb[2]));
+        if (fabs(B) < 2147483648.0) {
+            bq = __double2ll_rn(B * 4294967296.0);  // B to 2^-32 (exact scaling)
+            bi = static_cast<int32_t>(bq >> 32);
+            bf = static_cast<uint32_t>(bq);
+        } else if (isfinite(B)) {
+            flag = true;
         }
-        r[d] = static_cast<uint32_t>(bi) + 0x80000000u;
-        r[4 + d] = bf;
-        r[9 + d] = __float_as_uint(static_cast<float>(bi));
-        small = small && bi < kFxSmallBI && bi > -kFxSmallBI;
     }
-    double w[3] = {0.0, 0.0, 0.0};
-    if (incompr) {   // projector as the reference forms it (src/field.rs:138-152)
-        double kk = 0.0;
-        for (int d = 0; d < dim; ++d) kk = __dadd_rn(kk, __dmul_rn(k[d], k[d]));
-        const double k_2 = __ddiv_rn(k[0], kk);
-        w[0] = __dadd_rn(1.0, -__dmul_rn(k[0], k_2));
-        w[1] = -__dmul_rn(k[1], k_2);
-        w[2] = -__dmul_rn(k[2], k_2);
-    }
-    r[3] = __float_as_uint(__double2float_rn(w[0]));
-    r[7] = __float_as_uint(__double2float_rn(w[1]));
-    r[8] = __float_as_uint(__double2float_rn(w[2]));
-    if (!small) atomicOr(small_word, 1ull);
-    for (int q = 12; q < kFxTab; ++q) r[q] = 0u;
-    // phi mod 2^32, exactly (0 <= phi < 3 2^32, a multiple of 1/2)
-    phi -= 4294967296.0 * floor(phi * 2.3283064365386963e-10);
-    // T[m] = (z1 - i z2) e^{-2 pi i phi / 2^32} e^{2 pi i m / 16}: one FP64
-    // sincos for the mode's rotation, the sixteenth turns from a table (FP64
-    // products, a few FP64 ulps)
-    double s0, c0;
-    sincos(phi * -1.4629180792671596e-09, &s0, &c0);
-    const double ar = z1 * c0 + z2 * s0, ai = z1 * s0 - z2 * c0;   // (z1 - i z2) e^{i a}
+    if (live && flag && range_flag) *range_flag = 1;
+    const bool finite = isfinite(z1) && isfinite(z2) && isfinite(k);
+    const bool all_finite = ((__ballot_sync(0xffffffffu, !finite) >> g0) & 15u) == 0;
+    const bool large = live && !(bi < kFxSmallBI && bi > -kFxSmallBI);   // not every |BI| < 2^20
+    if (((__ballot_sync(0xffffffffu, large) >> g0) & 15u) && l == 0) atomicOr(small_word, 1ull);
+    // B 2^31 mod 2^32, what the offset 2^60 of X adds to theta, of all
+    // dimensions: in units of 2^-33 turn the low 33 bits of their bq
+    uint64_t turn = static_cast<uint64_t>(bq);
+    turn += __shfl_xor_sync(0xffffffffu, turn, 1);
+    turn += __shfl_xor_sync(0xffffffffu, turn, 2);
+    // T[m] = (z1 - i z2) e^{2 pi i (m / 16 - phi)}
+    int64_t co, si;
+    cis_fine((static_cast<uint64_t>(l) << 60) - (turn << 31) + kFineOffset, &co, &si);
+    const double c0 = static_cast<double>(co) * 0x1p-62, s0 = static_cast<double>(si) * 0x1p-62;
     const float nanf_ = __int_as_float(0x7fffffff);
-#pragma unroll
-    for (int m = 0; m < 16; ++m) {
-        const double cm = kSixteenthCos[m], sm = kSixteenthCos[(m + 12) & 15];   // sin = cos(. - 1/4)
-        const float tr = __double2float_rn(ar * cm - ai * sm);
-        const float ti = __double2float_rn(ar * sm + ai * cm);
-        r[kFxTab + 2 * m] = __float_as_uint(finite ? tr : nanf_);
-        r[kFxTab + 2 * m + 1] = __float_as_uint(finite ? ti : nanf_);
+    const float tr = all_finite ? __double2float_rn(z1 * c0 + z2 * s0) : nanf_;
+    const float ti = all_finite ? __double2float_rn(z1 * s0 - z2 * c0) : nanf_;
+    double w = 0.0;
+    if (incompr) {   // projector as the reference forms it (src/field.rs:138-152)
+        const double k0 = __shfl_sync(0xffffffffu, k, g0), k1 = __shfl_sync(0xffffffffu, k, g0 + 1),
+                     k2 = __shfl_sync(0xffffffffu, k, g0 + 2);
+        double kk = __dadd_rn(__dmul_rn(k0, k0), __dmul_rn(k1, k1));
+        if (dim > 2) kk = __dadd_rn(kk, __dmul_rn(k2, k2));
+        w = -__dmul_rn(k, __ddiv_rn(k0, kk));
+        if (l == 0) w = __dadd_rn(1.0, w);
     }
+    const uint32_t wf = __float_as_uint(__double2float_rn(w));
+    const uint32_t bif = __float_as_uint(static_cast<float>(bi)), bib = static_cast<uint32_t>(bi) + 0x80000000u;
+    // words 0..3 by lane 0, 4..7 by lane 1, 8..11 by lane 2
+    auto of = [&](uint32_t v, int d) { return __shfl_sync(0xffffffffu, v, g0 + d); };
+    const uint32_t w0 = of(wf, 0), w1 = of(wf, 1), w2 = of(wf, 2);
+    const uint4 h0 = make_uint4(of(bib, 0), of(bib, 1), of(bib, 2), w0);
+    const uint4 h1 = make_uint4(of(bf, 0), of(bf, 1), of(bf, 2), w1);
+    const uint4 h2 = make_uint4(w2, of(bif, 0), of(bif, 1), of(bif, 2));
+    if (!live) return;
+    if (l < 3) reinterpret_cast<uint4 *>(r)[l] = l == 0 ? h0 : l == 1 ? h1 : h2;
+    float2 *t = reinterpret_cast<float2 *>(r + kFxTab) + l;
+    t[0] = make_float2(tr, ti);
+    t[4] = make_float2(-ti, tr);
+    t[8] = make_float2(-tr, -ti);
+    t[12] = make_float2(ti, -tr);
 }
 
-// One warp of modes per block.  A record is one thread's dependent chain of
-// FP64 operations (about 13 us on GB300 for any number of modes per warp),
-// so the kernel takes that latency once.  Each block first reduces the range
-// kernel's per-block maxima; block 0 stores them as the range words of the
-// sums.
-constexpr int kFxModeThreads = 32;
+// Records of modes [j0, j0 + nc).  Each block first reduces the range kernel's
+// per-block maxima; block 0 stores them as the range words of the sums.
+constexpr int kFxModeThreads = 128, kFxModeLanes = 4;
 __global__ void __launch_bounds__(kFxModeThreads)
 fx_mode_kernel(const double *__restrict__ cov, const double *__restrict__ z1,
                const double *__restrict__ z2, int dim, int64_t n_modes, int64_t j0, int64_t nc,
                int incompr, const unsigned long long *__restrict__ range_part, int range_blocks,
                unsigned long long *maxbits, uint32_t *__restrict__ rec, int *range_flag) {
+    __shared__ unsigned long long warp_max[kFxModeThreads / 32][3];
+    wait_previous();
     // the mode's inputs first (they may come over the host link), so that
     // their latency overlaps the reduction of the range words
-    after_previous();
-    const int64_t jl = static_cast<int64_t>(blockIdx.x) * kFxModeThreads + threadIdx.x;
+    const int64_t jl = (static_cast<int64_t>(blockIdx.x) * kFxModeThreads + threadIdx.x) / kFxModeLanes;
     const int64_t j = j0 + jl;
-    const bool mine = jl < nc;
-    double k[3] = {0.0, 0.0, 0.0}, z1j = 0.0, z2j = 0.0;
-    if (mine) {
-        for (int d = 0; d < dim && d < 3; ++d) k[d] = cov[d * n_modes + j];
-        z1j = z1[j];
-        z2j = z2[j];
-    }
+    const bool live = jl < nc;
+    const int l = threadIdx.x & 3;
+    const double k = live && l < dim ? cov[l * n_modes + j] : 0.0;
+    const double z1j = live ? z1[j] : 0.0, z2j = live ? z2[j] : 0.0;
     unsigned long long mb[3] = {0ull, 0ull, 0ull};
     for (int b = threadIdx.x; b < range_blocks; b += kFxModeThreads)
         for (int d = 0; d < dim && d < 3; ++d)
             mb[d] = max(mb[d], range_part[3 * static_cast<int64_t>(b) + d]);
 #pragma unroll
-    for (int d = 0; d < 3; ++d)
+    for (int d = 0; d < 3; ++d) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mb[d] = max(mb[d], __shfl_xor_sync(0xffffffffu, mb[d], o));
+        if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5][d] = mb[d];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int w = 0; w < kFxModeThreads / 32; ++w) mb[d] = max(mb[d], warp_max[w][d]);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         maxbits[0] = mb[0];
         maxbits[1] = mb[1];
         maxbits[2] = mb[2];
     }
-    if (!mine) return;
-    fx_mode_entry(k, z1j, z2j, dim, incompr, mb, maxbits + 3, rec + jl * kFxRecWords, range_flag);
+    fx_mode_entry(live, k, z1j, z2j, dim, incompr, mb, maxbits + 3, rec + jl * kFxRecWords, range_flag);
+    next_may_start();
 }
 
 // Knuth's TwoSum: (hi, lo) += a
@@ -698,30 +702,36 @@ batch_fx_range_kernel(const BatchItem *__restrict__ items, unsigned long long *m
                   maxbits + 4 * blockIdx.x);
 }
 
-// Records of every item, one thread per mode (Fourier factor folded into z1,
-// z2 first).
-__global__ void batch_fx_table_kernel(const BatchItem *__restrict__ items,
-                                      const int64_t *__restrict__ prefix, int64_t n_items,
-                                      int64_t total, unsigned long long *maxbits,
-                                      uint32_t *__restrict__ rec, int *range_flag) {
-    const int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (g >= total) return;
-    int64_t lo = 0, hi = n_items - 1;
+// Records of every item, four lanes per mode (Fourier factor folded into z1, z2
+// first).
+constexpr int kBatchTableThreads = 128;
+__global__ void __launch_bounds__(kBatchTableThreads)
+batch_fx_table_kernel(const BatchItem *__restrict__ items,
+                      const int64_t *__restrict__ prefix, int64_t n_items,
+                      int64_t total, unsigned long long *maxbits,
+                      uint32_t *__restrict__ rec, int *range_flag) {
+    const int l = threadIdx.x & 3;
+    const int64_t g = (static_cast<int64_t>(blockIdx.x) * kBatchTableThreads + threadIdx.x) / kFxModeLanes;
+    const bool live = g < total;
+    int64_t lo = 0, hi = live ? n_items - 1 : 0;
     while (lo < hi) {
         const int64_t mid = (lo + hi + 1) >> 1;
         if (prefix[mid] <= g) lo = mid; else hi = mid - 1;
     }
     const BatchItem &it = items[lo];
     const int64_t j = g - it.mode_off;
-    double z1j = it.z1[j], z2j = it.z2[j];
-    if (it.sf) {
-        const double f = it.sf[j];
-        z1j = __dmul_rn(f, z1j);
-        z2j = __dmul_rn(f, z2j);
+    double k = 0.0, z1j = 0.0, z2j = 0.0;
+    if (live) {
+        z1j = it.z1[j];
+        z2j = it.z2[j];
+        if (it.sf) {
+            const double f = it.sf[j];
+            z1j = __dmul_rn(f, z1j);
+            z2j = __dmul_rn(f, z2j);
+        }
+        if (l < it.dim) k = it.cov[l * it.n_modes + j];
     }
-    double k[3] = {0.0, 0.0, 0.0};
-    for (int d = 0; d < it.dim && d < 3; ++d) k[d] = it.cov[d * it.n_modes + j];
-    fx_mode_entry(k, z1j, z2j, it.dim, it.incompr, maxbits + 4 * lo, maxbits + 4 * lo + 3,
+    fx_mode_entry(live, k, z1j, z2j, it.dim, it.incompr, maxbits + 4 * lo, maxbits + 4 * lo + 3,
                   rec + g * kFxRecWords, range_flag);
 }
 
@@ -853,7 +863,7 @@ int mixed_fx_run(DeviceCtx &ctx, const PlainArgs &a, int *range_flag, cudaStream
         if (nc <= 0) return GSC_OK;
         TimedLaunch tl(st);
         tl.begin(K_MIXED_MODES);
-        GSC_CUDA(launch_after(fx_mode_kernel, dim3(static_cast<unsigned>((nc + kFxModeThreads - 1) / kFxModeThreads)),
+        GSC_CUDA(launch_after(fx_mode_kernel, dim3(static_cast<unsigned>((nc * kFxModeLanes + kFxModeThreads - 1) / kFxModeThreads)),
                               dim3(kFxModeThreads), 0, st, a.cov, a.z1, a.z2, static_cast<int>(dim), N, j0, nc,
                               a.incompr ? 1 : 0, range_part, static_cast<int>(rb), maxbits, rec, range_flag));
         tl.end();
@@ -945,7 +955,8 @@ int batch_fx_tables(const BatchItem *items, const int64_t *mode_prefix, int64_t 
     batch_fx_range_kernel<<<dim3(static_cast<unsigned>(n_items), kBatchRangeBlocks),
                             kBatchRangeThreads, 0, st>>>(items, maxbits);
     if (total_modes > 0)
-        batch_fx_table_kernel<<<static_cast<unsigned>((total_modes + 127) / 128), 128, 0, st>>>(
+        batch_fx_table_kernel<<<static_cast<unsigned>((total_modes * kFxModeLanes + kBatchTableThreads - 1) / kBatchTableThreads),
+                                kBatchTableThreads, 0, st>>>(
             items, mode_prefix, n_items, total_modes, maxbits, rec, range_flag);
     tl.end();
     GSC_CUDA(cudaGetLastError());
