@@ -272,7 +272,7 @@ __device__ __forceinline__ double scale_pow2(double x, int n) {
 // 0): a first angle in FP32, its cosine and sine in 64 bits, then the remaining
 // rotation d (1e-7 rad) from the cross product.  An FP64 atan2 and hypot would
 // be a longer chain, and less exact.
-__device__ __forceinline__ void mode_angle(double z1, double z2, const CosTable *tab, double *amp,
+__device__ __forceinline__ void mode_angle(double z1, double z2, double *amp,
                                            int *ez, uint64_t *beta) {
     *amp = 0.0;
     *ez = 0;
@@ -284,7 +284,7 @@ __device__ __forceinline__ void mode_angle(double z1, double z2, const CosTable 
     const float t = atan2f(static_cast<float>(f2), static_cast<float>(f1)) * 0.15915494f;   // turns
     const uint64_t b = static_cast<uint64_t>(__float2ll_rn(t * 1099511627776.0f)) << 24;
     int64_t c, s;
-    cis_fine(b + kFineOffset, tab, &c, &s);
+    cis_fine(b + kFineOffset, &c, &s);
     const double along = static_cast<double>(__mul64hi(f1, c) + __mul64hi(f2, s));    // units 2^-60
     const double across = static_cast<double>(__mul64hi(f2, c) - __mul64hi(f1, s));
     // across / along to 2^-45 of it: an FP32 reciprocal and one Newton step

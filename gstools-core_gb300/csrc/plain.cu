@@ -83,7 +83,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void rec_group(const double *__restrict__ cov, int64_t n_modes, int dim,
                                           int64_t j, bool live, double z1, double z2, int incompr,
-                                          double *__restrict__ r, const CosTable *tab) {
+                                          double *__restrict__ r) {
     double k[3] = {0.0, 0.0, 0.0}, w[3] = {0.0, 0.0, 0.0};
     if (live)
         for (int d = 0; d < dim && d < 3; ++d) k[d] = cov[d * n_modes + j];
@@ -101,7 +101,7 @@ __device__ __forceinline__ void rec_group(const double *__restrict__ cov, int64_
     uint64_t beta = 0;
     double amp = 0.0;                                            // A 2^-ez
     int ez = 0;
-    if (regular) mode_angle(z1, z2, tab, &amp, &ez, &beta);
+    if (regular) mode_angle(z1, z2, &amp, &ez, &beta);
     const int nout = incompr ? dim : 1;
     double a[3] = {incompr ? amp * w[0] : amp, amp * w[1], amp * w[2]};
     double scale[3] = {0.0, 0.0, 0.0};
@@ -149,18 +149,13 @@ __global__ void __launch_bounds__(kThreads)
 plain_rec_kernel(const double *__restrict__ cov, const double *__restrict__ z1,
                  const double *__restrict__ z2, int dim, int64_t n_modes, int64_t j0, int64_t nc,
                  int incompr, double *__restrict__ rec, const int *__restrict__ run_if) {
-    __shared__ CosTable tab;
-    if (run_if) {
-        after_previous();
-        if (*run_if == 0) return;            // a predicated launch that is not wanted
-    }
-    fill_cos_table(&tab, threadIdx.x, kThreads);
-    __syncthreads();
-    after_previous();
+    wait_previous();
+    if (run_if && *run_if == 0) return;      // a predicated launch that is not wanted
     const int64_t jl = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x, j = j0 + jl;
     const bool live = jl < nc;
     const double a = live ? z1[j] : 0.0, b = live ? z2[j] : 0.0;
-    rec_group(cov, n_modes, dim, j, live, a, b, incompr, rec + jl * kRec, &tab);
+    rec_group(cov, n_modes, dim, j, live, a, b, incompr, rec + jl * kRec);
+    next_may_start();
 }
 
 // Records of every item of a batch: the warps of column blockIdx.y walk the
@@ -168,9 +163,6 @@ plain_rec_kernel(const double *__restrict__ cov, const double *__restrict__ z1,
 // and z2 first.
 __global__ void __launch_bounds__(kThreads)
 batch_rec_kernel(const BatchItem *__restrict__ items, int64_t n_items, double *__restrict__ rec) {
-    __shared__ CosTable tab;
-    fill_cos_table(&tab, threadIdx.x, kThreads);
-    __syncthreads();
     for (int64_t i = blockIdx.y; i < n_items; i += gridDim.y) {
         const BatchItem &it = items[i];
         const int64_t groups = (it.n_modes + kGroup - 1) / kGroup;
@@ -185,7 +177,7 @@ batch_rec_kernel(const BatchItem *__restrict__ items, int64_t n_items, double *_
                 b = __dmul_rn(f, b);
             }
             rec_group(it.cov, it.n_modes, it.dim, j, live, a, b, it.incompr,
-                      rec + (it.mode_off + j) * kRec, &tab);
+                      rec + (it.mode_off + j) * kRec);
         }
     }
 }

@@ -113,9 +113,6 @@ __device__ __forceinline__ int ceil_exponent(double x) {
 // z1 + i z2 of every mode as amplitude and angle, projector weights and the
 // exponents of the largest.
 __global__ void __launch_bounds__(128) sl_modes_kernel(SlTab t) {
-    __shared__ CosTable tab;
-    fill_cos_table(&tab, threadIdx.x, 128);
-    __syncthreads();
     after_previous();
     const int j = blockIdx.x * 128 + threadIdx.x;
     const bool live = j < t.n_modes;
@@ -142,7 +139,7 @@ __global__ void __launch_bounds__(128) sl_modes_kernel(SlTab t) {
         m.amp = 0.0;
         m.beta = 0;
         if (!bad) {
-            mode_angle(z1, z2, &tab, &m.amp, &m.ez, &m.beta);
+            mode_angle(z1, z2, &m.amp, &m.ez, &m.beta);
             if (m.amp > 0.0) {
                 m.ea = m.ez + ceil_exponent(m.amp);            // A <= 2^ea
                 bad = m.ea < -900 || m.ea > 900;
@@ -201,9 +198,6 @@ __device__ __forceinline__ uint32_t chunk_offset(int r, int c) {
 constexpr int kTabThreads = 256;
 __global__ void __launch_bounds__(kTabThreads)
 sl_tables_kernel(SlTab t, int64_t n_g, int64_t n_b, int64_t n_s) {
-    __shared__ CosTable tab;
-    fill_cos_table(&tab, threadIdx.x, kTabThreads);
-    __syncthreads();
     after_previous();
     const int np = t.kb * kKbModes;
     const int ew = top_exponent(t.words[1]);
@@ -232,7 +226,7 @@ sl_tables_kernel(SlTab t, int64_t n_g, int64_t n_b, int64_t n_s) {
                 if (comp < t.ncomp && jl < t.nj) {
                     const SlMode &m = t.modes[j];
                     int64_t co, si;
-                    cis_fine(fraction(t.dim - 1, j, t.ax_n[n]) + kFineOffset, &tab, &co, &si);
+                    cis_fine(fraction(t.dim - 1, j, t.ax_n[n]) + kFineOffset, &co, &si);
                     const int g = t.incompr ? top_exponent(t.words[2 + comp]) : 0;
                     const int64_t wf = __double2ll_rn(scale_pow2(m.w[comp], 62 - g - mode_shift(m, ew)));
                     re = __mul64hi(wf, co);
@@ -253,7 +247,7 @@ sl_tables_kernel(SlTab t, int64_t n_g, int64_t n_b, int64_t n_s) {
             longlong2 v = make_longlong2(0, 0);
             if (jl < t.nj) {
                 int64_t co, si;
-                cis_fine(fraction(t.dim - 2, t.j0 + jl, t.ax_m[m]) + kFineOffset, &tab, &co, &si);
+                cis_fine(fraction(t.dim - 2, t.j0 + jl, t.ax_m[m]) + kFineOffset, &co, &si);
                 v = make_longlong2(co, si);
             }
             t.btab[i] = v;
@@ -269,7 +263,7 @@ sl_tables_kernel(SlTab t, int64_t n_g, int64_t n_b, int64_t n_s) {
                 uint64_t th = kFineOffset - m.beta;
                 if (t.dim == 3) th += fraction(0, j, t.ax_b[b]);
                 int64_t co, si;
-                cis_fine(th, &tab, &co, &si);
+                cis_fine(th, &co, &si);
                 const int64_t a = __double2ll_rn(scale_pow2(m.amp, m.ez - ew + mode_shift(m, ew) + 62));
                 v = make_longlong2(__mul64hi(a, co) << 2, __mul64hi(a, si) << 2);
             }
