@@ -47,6 +47,7 @@
 #include <algorithm>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 
 #include "dfturns.cuh"
 #include "internal.h"
@@ -1519,18 +1520,39 @@ sep_x5_kernel(const __grid_constant__ CUtensorMap out_map, const X5Params xp) {
                 // within 2^24 counts
                 const float lim = 16777216.0f * cnt_unit;
                 bool over = false;
+                // eight columns' loads of every part in flight at a time: one
+                // column after the other, each waited for, took longer than the
+                // rest of a small call
+                constexpr int kBatch = 8;
+                static_assert(L::HC % kBatch == 0, "columns per batch");
+                auto add_parts = [&](auto parts) {
+                    constexpr int K = decltype(parts)::value;
 #pragma unroll
-                for (int c = 0; c < L::HC; ++c) {
-                    float a = __ldcg(col0 + c * BM), mm = __ldcg(colm + c * BM);
+                    for (int c0 = 0; c0 < L::HC; c0 += kBatch) {
+                        float a[kBatch][K], mm[kBatch][K];
 #pragma unroll
-                    for (int k = 1; k < kMaxSplit; ++k)
-                        if (k < ks) {
-                            a += __ldcg(col0 + (k * BNX + c) * BM);
-                            mm += __ldcg(colm + (k * BNX + c) * BM);
-                            over = over || fabsf(mm) > lim;
+                        for (int c = 0; c < kBatch; ++c)
+#pragma unroll
+                            for (int k = 0; k < K; ++k) {
+                                a[c][k] = __ldcg(col0 + (k * BNX + c0 + c) * BM);
+                                mm[c][k] = __ldcg(colm + (k * BNX + c0 + c) * BM);
+                            }
+#pragma unroll
+                        for (int c = 0; c < kBatch; ++c) {
+#pragma unroll
+                            for (int k = 1; k < K; ++k) {
+                                a[c][0] += a[c][k];
+                                mm[c][0] += mm[c][k];
+                                over = over || fabsf(mm[c][0]) > lim;
+                            }
+                            tot[c0 + c] = fixed(mm[c][0], a[c][0]);
                         }
-                    tot[c] = fixed(mm, a);
-                }
+                    }
+                };
+                static_assert(kMaxSplit == 4, "parts of a split tile");
+                if (ks == 2) add_parts(std::integral_constant<int, 2>{});
+                else if (ks == 3) add_parts(std::integral_constant<int, 3>{});
+                else add_parts(std::integral_constant<int, 4>{});
                 if (over && row_ok) {
                     *xp.bound_flag = 1;
                     if (xp.bound_sticky) *xp.bound_sticky = 1;
