@@ -47,7 +47,6 @@
 #include <algorithm>
 #include <cmath>
 #include <mutex>
-#include <type_traits>
 
 #include "dfturns.cuh"
 #include "internal.h"
@@ -884,13 +883,12 @@ struct X5Params {
     // Tail split: tiles [0, full_tiles) run whole, one per CTA; each of the
     // n_split later tiles runs as ksplit CTAs (the launch's first n_split *
     // ksplit blocks) over consecutive parts of its k-blocks, whose
-    // FP32 partials meet in `ws` ([slot][part][column][row]); the last part
-    // to finish (counted in ws_cnt[slot]) adds them in part order and stores.
+    // FP32 partials go to `ws` ([slot][part][column][row]), where
+    // sep_x5_join_kernel adds them in part order.
     int tile0;               // first tile of this launch (launches of wave-sized row ranges)
     int full_tiles, ksplit, n_split;
     float *ws;               // cross totals of the parts
     float *ws_main;          // exact main sums of the parts (same layout)
-    int *ws_cnt;
     // 2 or 3: the output is written by tiled bulk stores through the kernel's
     // tensor map of that rank ((nn, rows) or (nn, rows, components));
     // 0: by plain stores
@@ -944,9 +942,10 @@ struct X5Layout {
     static constexpr size_t SMEM = DATA + 1024 + 256;
     static constexpr int HC = BNX / 2;                   // columns per worker half
     // setmaxnreg split: workers hold HC FP32 totals; the narrower tile leaves
-    // the control warps room (chosen where ptxas reports no spills)
-    static constexpr int WORK_REGS = BNX == 256 ? 216 : 200;
-    static constexpr int CTRL_REGS = BNX == 256 ? 48 : 80;
+    // the control warps room (192^3 x 2048 modes, incompressible: 711 us with
+    // 184 / 136, 724 with 200 / 104, 735 with 200 / 80, which spill)
+    static constexpr int WORK_REGS = BNX == 256 ? 216 : 184;
+    static constexpr int CTRL_REGS = BNX == 256 ? 48 : 136;
     static_assert(4 * 32 * (2 * WORK_REGS + CTRL_REGS) <= X5_THREADS * X5_LAUNCH_REGS,
                   "setmaxnreg split exceeds the registers the block is launched with");
     static_assert(OFF_G2 % 1024 == 0 && OFF_B % 1024 == 0 && STAGE % 1024 == 0,
@@ -974,6 +973,16 @@ __device__ __forceinline__ void slice3x2(float2 v, float ls, float lu, float ku,
     w3 = *reinterpret_cast<const uint32_t *>(&h3);
 }
 
+// An output as a 32-bit integer of 1/64 counts (its bits): the exact main sum
+// and the rounded cross total.  A NaN or infinite sum (NaN inputs) becomes the
+// sentinel -2^31, which no finite sum reaches (|main| < 2^30, the cross total
+// far less).
+__device__ __forceinline__ float x5_counts(float mainv, float crossv, float to_t) {
+    const bool finite = fabsf(mainv) <= 3.0e38f && fabsf(crossv) <= 3.0e38f;
+    return __int_as_float(finite ? __float2int_rn(mainv * to_t) + __float2int_rn(crossv * to_t)
+                                 : static_cast<int>(0x80000000u));
+}
+
 template <int BNX, bool SPLIT>
 __global__ void __launch_bounds__(X5_THREADS, 1)
 sep_x5_kernel(const __grid_constant__ CUtensorMap out_map, const X5Params xp) {
@@ -999,7 +1008,6 @@ sep_x5_kernel(const __grid_constant__ CUtensorMap out_map, const X5Params xp) {
     uint64_t *b_empty = bars + 16;              // [3] workers -> copy warp (8 arrivals)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 19);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    volatile int *last_part = reinterpret_cast<volatile int *>(tmem_slot + 2);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Rows are the nb * nm (x-slice, y) pairs taken in order, so a 128-row
@@ -1384,13 +1392,6 @@ sep_x5_kernel(const __grid_constant__ CUtensorMap out_map, const X5Params xp) {
         // the exponent.  No FP32 rounding at the field's magnitude remains.
         const float to_t = xp.wnorm[6];
         const int qexp = static_cast<int>(xp.wnorm[7]);
-        // a NaN or infinite sum (NaN inputs) leaves as the sentinel -2^31,
-        // which no finite sum reaches (|main| < 2^30, the cross total far less)
-        auto fixed = [&](float mainv, float crossv) -> float {
-            const bool finite = fabsf(mainv) <= 3.0e38f && fabsf(crossv) <= 3.0e38f;
-            return __int_as_float(finite ? __float2int_rn(mainv * to_t) + __float2int_rn(crossv * to_t)
-                                         : static_cast<int>(0x80000000u));
-        };
         auto to_f64 = [&](float bits) -> double { return i32_to_f64_pow2(__float_as_int(bits), qexp); };
         float *trf = reinterpret_cast<float *>(smem) + warp * (32 * 33);
         // output offset of row (warp's first row) + R; the warp's first row
@@ -1403,24 +1404,31 @@ sep_x5_kernel(const __grid_constant__ CUtensorMap out_map, const X5Params xp) {
             }
             return static_cast<int64_t>(bs) * p.batch_stride + static_cast<int64_t>(ms) * p.row_stride;
         };
-        // column group g: tot[32g .. 32g+31] += the cross accumulator's last
-        // chunk, then each main sum with its cross total goes to `use` (in
-        // halves of 16, to keep registers free)
+        // Column group g, one after the other in a loop that is not unrolled:
+        // its totals are the first 32, and the others move down afterwards.
+        // (Unrolled, the epilogue is straight-line code of tens of KB, whose
+        // fetch took longer than its work where an SM runs one tile.)
+        // tot[0 .. 31] += the cross accumulator's last chunk, then each main
+        // sum goes to `use` (in halves of 16, to keep registers free)
         auto read_group = [&](int g, auto &&use) {
             uint32_t v[32];
             __syncwarp();
             tmem_ld32(t_cross + lane_off + L::HC * h + 32 * g, v);
             tmem_ld_wait();
 #pragma unroll
-            for (int t = 0; t < 32; ++t) tot[32 * g + t] += __uint_as_float(v[t]);
+            for (int t = 0; t < 32; ++t) tot[t] += __uint_as_float(v[t]);
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
                 uint32_t mv[16];
                 tmem_ld16(t_main + lane_off + L::HC * h + 32 * g + 16 * hf, mv);
                 tmem_ld_wait();
 #pragma unroll
-                for (int t = 0; t < 16; ++t) use(32 * g + 16 * hf + t, __uint_as_float(mv[t]));
+                for (int t = 0; t < 16; ++t) use(16 * hf + t, __uint_as_float(mv[t]));
             }
+        };
+        auto next_group = [&]() {
+#pragma unroll
+            for (int t = 0; t + 32 < L::HC; ++t) tot[t] = tot[t + 32];
         };
         auto store_group = [&](int g) {
             const int rows = max(0, min(32, rows_valid - 32 * q));
@@ -1440,7 +1448,7 @@ sep_x5_kernel(const __grid_constant__ CUtensorMap out_map, const X5Params xp) {
                 for (int hb = 0; hb < 2; ++hb)
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
-                        const int t = 32 * g + 16 * hb + 2 * c;
+                        const int t = 16 * hb + 2 * c;
                         *reinterpret_cast<double2 *>(bx + hb * 4096 + lane * 128 + ((c ^ (lane & 7)) << 4)) =
                             make_double2(to_f64(tot[t]), to_f64(tot[t + 1]));
                     }
@@ -1464,7 +1472,7 @@ sep_x5_kernel(const __grid_constant__ CUtensorMap out_map, const X5Params xp) {
                 // column per lane: 256 contiguous bytes per row and store
                 __syncwarp();
 #pragma unroll
-                for (int t = 0; t < 32; ++t) trf[lane * 33 + t] = tot[32 * g + t];
+                for (int t = 0; t < 32; ++t) trf[lane * 33 + t] = tot[t];
                 __syncwarp();
                 const int gn = gc + lane;
                 const int bs0 = static_cast<int>(rq / p.nm), ms0 = static_cast<int>(rq % p.nm);
@@ -1475,91 +1483,27 @@ sep_x5_kernel(const __grid_constant__ CUtensorMap out_map, const X5Params xp) {
                 }
             }
         };
-        if (!split) {
-            if (ok) {
-                tc_fence_after();
-#pragma unroll
-                for (int g = 0; g < L::HC / 32; ++g) {
-                    read_group(g, [&](int c, float mainv) { tot[c] = fixed(mainv, tot[c]); });
-                    store_group(g);
-                }
-                __syncwarp();
+        if (ok) tc_fence_after();
+        if (ok && !split) {
+#pragma unroll 1
+            for (int g = 0; g < L::HC / 32; ++g) {
+                read_group(g, [&](int c, float mainv) { tot[c] = x5_counts(mainv, tot[c], to_t); });
+                store_group(g);
+                next_group();
             }
-        } else if (SPLIT) {
-            // a split tile: write this part's main sums and cross totals,
-            // count the parts, and the last part adds all of them in part
-            // order (the result does not depend on which part finishes
-            // last; the main sums add exactly), then stores as above
-            const int slot = tile - xp.tile0 - xp.full_tiles, ks = xp.ksplit;
-            const int64_t slot_off = static_cast<int64_t>(slot) * ks * BNX * BM;
-            // this thread's column c of part k sits at col0[(k * BNX + c) * BM]
-            const int64_t c_off = static_cast<int64_t>(L::HC * h) * BM + r;
-            float *col0 = xp.ws + slot_off + c_off;
-            float *colm = xp.ws_main + slot_off + c_off;
-            if (ok) {
-                tc_fence_after();
-                float *wm = colm + static_cast<int64_t>(part) * BNX * BM;
+            __syncwarp();
+        } else if (SPLIT && ok) {
+            // a part of a split tile: its main sums and cross totals go to the
+            // workspace, column c of part k at (k * BNX + c) * BM + row
+            const int64_t at = (static_cast<int64_t>(tile - xp.tile0 - xp.full_tiles) * xp.ksplit + part) * BNX * BM +
+                               static_cast<int64_t>(L::HC * h) * BM + r;
+#pragma unroll 1
+            for (int g = 0; g < L::HC / 32; ++g) {
+                float *wm = xp.ws_main + at + 32 * g * BM, *wp = xp.ws + at + 32 * g * BM;
+                read_group(g, [&](int c, float mainv) { wm[c * BM] = mainv; });
 #pragma unroll
-                for (int g = 0; g < L::HC / 32; ++g)
-                    read_group(g, [&](int c, float mainv) { wm[c * BM] = mainv; });
-                float *wp = col0 + static_cast<int64_t>(part) * BNX * BM;
-#pragma unroll
-                for (int c = 0; c < L::HC; ++c) wp[c * BM] = tot[c];
-            }
-            __threadfence();
-            asm volatile("bar.sync 1, 256;" ::: "memory");      // the 256 worker threads
-            if (threadIdx.x == 0)
-                *last_part = (!*abort_flag && atomicAdd(xp.ws_cnt + slot, 1) == ks - 1) ? 1 : 0;
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (ok && *last_part) {
-                __threadfence();
-                if (threadIdx.x == 0) xp.ws_cnt[slot] = 0;          // ready for the next launch
-                // every part (this one included) is read back from the
-                // workspace, so the sums need no second register array; the
-                // parts' main sums add exactly while the running total stays
-                // within 2^24 counts
-                const float lim = 16777216.0f * cnt_unit;
-                bool over = false;
-                // eight columns' loads of every part in flight at a time: one
-                // column after the other, each waited for, took longer than the
-                // rest of a small call
-                constexpr int kBatch = 8;
-                static_assert(L::HC % kBatch == 0, "columns per batch");
-                auto add_parts = [&](auto parts) {
-                    constexpr int K = decltype(parts)::value;
-#pragma unroll
-                    for (int c0 = 0; c0 < L::HC; c0 += kBatch) {
-                        float a[kBatch][K], mm[kBatch][K];
-#pragma unroll
-                        for (int c = 0; c < kBatch; ++c)
-#pragma unroll
-                            for (int k = 0; k < K; ++k) {
-                                a[c][k] = __ldcg(col0 + (k * BNX + c0 + c) * BM);
-                                mm[c][k] = __ldcg(colm + (k * BNX + c0 + c) * BM);
-                            }
-#pragma unroll
-                        for (int c = 0; c < kBatch; ++c) {
-#pragma unroll
-                            for (int k = 1; k < K; ++k) {
-                                a[c][0] += a[c][k];
-                                mm[c][0] += mm[c][k];
-                                over = over || fabsf(mm[c][0]) > lim;
-                            }
-                            tot[c0 + c] = fixed(mm[c][0], a[c][0]);
-                        }
-                    }
-                };
-                static_assert(kMaxSplit == 4, "parts of a split tile");
-                if (ks == 2) add_parts(std::integral_constant<int, 2>{});
-                else if (ks == 3) add_parts(std::integral_constant<int, 3>{});
-                else add_parts(std::integral_constant<int, 4>{});
-                if (over && row_ok) {
-                    *xp.bound_flag = 1;
-                    if (xp.bound_sticky) *xp.bound_sticky = 1;
-                }
-#pragma unroll
-                for (int g = 0; g < L::HC / 32; ++g) store_group(g);
-                __syncwarp();
+                for (int c = 0; c < 32; ++c) wp[c * BM] = tot[c];
+                next_group();
             }
         }
     }
@@ -1570,6 +1514,64 @@ sep_x5_kernel(const __grid_constant__ CUtensorMap out_map, const X5Params xp) {
     __syncthreads();
     tc_fence_after();
     if (warp == kMmaWarpX5) tmem_dealloc(tmem, kTmemCols);
+}
+
+// Split tiles: the parts' sums added in part order (main sums exactly, while the
+// running total stays within 2^24 counts), converted and stored.  A block takes
+// 32 columns of a tile, a thread 16 of a row with all parts' loads in flight; the
+// doubles are turned around in shared memory.  As work of the last part's CTA
+// this took about 20 us of one SM a tile, most of it waiting for loads: at
+// 70^3 x 500 modes a third of the call.
+constexpr int kJoinColumns = 32, kJoinThreads = 2 * BM;
+template <int K>
+__global__ void __launch_bounds__(kJoinThreads) sep_x5_join_kernel(const X5Params xp, int bnx) {
+    __shared__ double tile_out[BM][kJoinColumns + 1];
+    after_previous();
+    if (*xp.bound_flag) return;          // the call is recomputed
+    const TcParams &p = xp.base;
+    const int tile = xp.tile0 + xp.full_tiles + static_cast<int>(blockIdx.y);
+    const int64_t r0 = static_cast<int64_t>(tile / p.n_tiles) * BM;
+    const int n0 = tile % p.n_tiles * bnx + static_cast<int>(blockIdx.x) * kJoinColumns;
+    if (n0 >= p.ncn) return;
+    const int rows = static_cast<int>(min(static_cast<int64_t>(BM), p.rows_total - r0));
+    const int r = threadIdx.x % BM, c0 = threadIdx.x / BM * (kJoinColumns / 2);
+    const int64_t at = (static_cast<int64_t>(blockIdx.y) * K * bnx + blockIdx.x * kJoinColumns + c0) * BM + r;
+    const float to_t = xp.wnorm[6], lim = 16777216.0f * (xp.wnorm[3] * 16.0f);
+    const int qexp = static_cast<int>(xp.wnorm[7]);
+    bool over = false;
+#pragma unroll
+    for (int b = 0; b < kJoinColumns / 2; b += 8) {
+        float a[8][K], m[8][K];
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const int64_t i = at + (static_cast<int64_t>(k) * bnx + b + c) * BM;
+                a[c][k] = __ldcg(xp.ws + i);
+                m[c][k] = __ldcg(xp.ws_main + i);
+            }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+#pragma unroll
+            for (int k = 1; k < K; ++k) {
+                a[c][0] += a[c][k];
+                m[c][0] += m[c][k];
+                over = over || fabsf(m[c][0]) > lim;
+            }
+            tile_out[r][c0 + b + c] = i32_to_f64_pow2(__float_as_int(x5_counts(m[c][0], a[c][0], to_t)), qexp);
+        }
+    }
+    if (over && r < rows) {
+        *xp.bound_flag = 1;
+        if (xp.bound_sticky) *xp.bound_sticky = 1;
+    }
+    __syncthreads();
+    const int c = threadIdx.x % kJoinColumns, gn = n0 + c;
+    if (gn >= p.ncn) return;
+    const int comp = gn / p.nn;
+    double *o = p.out + comp * p.comp_stride + (gn - comp * p.nn) + r0 * p.row_stride;   // (slice, y) rows are dense
+    for (int R = threadIdx.x / kJoinColumns; R < rows; R += kJoinThreads / kJoinColumns)
+        o[R * p.row_stride] = tile_out[R][c];
 }
 
 // ---------------------------------------------------------------------------
@@ -1734,11 +1736,10 @@ int sep_tc_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
     // cross totals and exact main sums of the split parts
     const size_t ws_half = static_cast<size_t>(n_split) * ksplit * bnx * BM * sizeof(float);
     const size_t ws_bytes = 2 * ws_half;
-    const size_t off_cnt = align_up(off_ws + ws_bytes, 1024);
     // x5: FP32 mode records and axis splits for the tables
     const int ax_off_m = dim == 3 ? nb : 0, ax_off_n = ax_off_m + nm;
     const int64_t n_ax = static_cast<int64_t>(ax_off_n) + nn;
-    const size_t off_l1 = align_up(off_cnt + static_cast<size_t>(n_split) * sizeof(int), 256);
+    const size_t off_l1 = align_up(off_ws + ws_bytes, 1024);
     const size_t off_mrec = align_up(off_l1 + (x5 ? sizeof(float) * static_cast<size_t>(KB) : 0), 1024);
     const size_t off_axs = align_up(off_mrec + (x5 ? sizeof(float) * kRecX5 * static_cast<size_t>(N) : 0), 1024);
     const size_t total = off_axs + (x5 ? sizeof(float2) * static_cast<size_t>(n_ax) : 0) + 256;
@@ -1865,7 +1866,6 @@ int sep_tc_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
         xp.bt = reinterpret_cast<const unsigned char *>(t.btab);
         xp.ws = reinterpret_cast<float *>(base + off_ws);
         xp.ws_main = reinterpret_cast<float *>(base + off_ws + ws_half);
-        xp.ws_cnt = reinterpret_cast<int *>(base + off_cnt);
         // The output (ncomp, rows, nn) is dense; tiled bulk stores write it
         // where its rows are 16-byte aligned and, for several components, no
         // 32-column group crosses from one component into the next.
@@ -1897,8 +1897,6 @@ int sep_tc_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
             xp.full_tiles = static_cast<int>(l.full_tiles);
             xp.ksplit = l.ksplit;
             xp.n_split = static_cast<int>(l.n_split);
-            if (l.n_split > 0)
-                GSC_CUDA(cudaMemsetAsync(xp.ws_cnt, 0, static_cast<size_t>(l.n_split) * sizeof(int), st));
             const unsigned g = static_cast<unsigned>(l.full_tiles + l.n_split * l.ksplit);
             if (bnx == 192 && l.n_split > 0) {
                 GSC_TRY((configure_x5<192, true>()));
@@ -1912,6 +1910,13 @@ int sep_tc_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
             } else {
                 GSC_TRY((configure_x5<256, false>()));
                 GSC_CUDA(launch_after(sep_x5_kernel<256, false>, dim3(g), dim3(X5_THREADS), X5Layout<256>::SMEM, st, om, xp));
+            }
+            if (l.n_split > 0) {
+                const auto join = l.ksplit == 2   ? sep_x5_join_kernel<2>
+                                  : l.ksplit == 3 ? sep_x5_join_kernel<3>
+                                                  : sep_x5_join_kernel<4>;
+                GSC_CUDA(launch_after(join, dim3(static_cast<unsigned>(bnx / kJoinColumns), static_cast<unsigned>(l.n_split)),
+                                      dim3(kJoinThreads), 0, st, xp, bnx));
             }
             GSC_CUDA(cudaGetLastError());
             if (a.on_rows)
