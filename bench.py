@@ -500,14 +500,14 @@ def run_ours(args, world, rank, local, wname, cpu_seconds, form_arg="auto"):
             e2e_structured = host_e2e(
                 scall, (w["cov"], w["z1"], w["z2"], w["axes"]), {"form": form}, reps, h2d,
                 f"gstools_core.{scall.__name__} (the axes; no reference counterpart)")
-            # default arguments: tolerance 1e-12, routed to the FP64 DMMA form
+            # default arguments: tolerance 1e-12, routed to the FP64 separable form
             dropin = host_e2e(call, (w["cov"], w["z1"], w["z2"], pos_h), {}, 2, h2d,
                               f"gstools_core.{call.__name__}(cov_samples, z1, z2, pos) with the "
                               "flattened meshgrid and default form / tolerance (1e-12)")
         del pos_h
 
     # ---- every value against an FP64 form on the GPU, itself checked
-    # against the oracle here: the FP64 DMMA contraction on grids, the plain
+    # against the oracle here: the FP64 contraction on grids, the plain
     # FP64 kernel on points (its timed step is the plain arm) --------------------
     full, plain = None, None
     ref_form = "sep_f64" if w["axes"] is not None else "plain"
@@ -522,7 +522,7 @@ def run_ours(args, world, rank, local, wname, cpu_seconds, form_arg="auto"):
             full = full_error(torch, out_d, rout)
             pin = check(rout)
             full["reference"] = (f"{ref_form} on the GPU ("
-                                 + ("FP64 DMMA contraction" if ref_form == "sep_f64"
+                                 + ("FP64 contraction" if ref_form == "sep_f64"
                                     else "plain FP64 kernel")
                                  + f"), itself {pin['max_abs_over_rms']:.2e} of RMS from the "
                                    f"oracle on {pin['points_checked']} points in this run")
@@ -1050,9 +1050,10 @@ def measured_peaks():
         return {}
 
 
-# FP64 pipe instructions per point*mode of the plain kernel's table path
-# (phase 2d-1, reduction + polynomials + table combine 12, accumulate 1 or d)
-PLAIN_FP64_OPS = {(1, False): 14, (2, False): 16, (3, False): 18, (2, True): 17, (3, True): 20}
+# FP64 pipe instructions per point*mode of the plain kernel: the first product
+# and the d - 1 sums of the phase, and half of the second products in 2-D (the
+# other products, the cosine and the sums run on the integer pipes)
+PLAIN_FP64_OPS = {(1, False): 1, (2, False): 2.5, (3, False): 3, (2, True): 2.5, (3, True): 3}
 # Instructions per point*mode of the mixed kernel (mixed_fx.cu) on the FMA
 # pipe, by kind, counted from the source for calls whose every |BI| < 2^20
 # (all workloads here): (high integer products, low integer products, FP32
@@ -1075,7 +1076,7 @@ MIXED_OPS = {(1, False): (1, 1, 11.375), (2, False): (2, 2, 12.375), (3, False):
 PROFILED_TRAFFIC = {
     ("sep_tc_f16x5", "c2"): (12.49e6 + 88.12e6, "profiles/sep_tc_f16x5_c2.md"),
     ("sep_tc_f16x5", "c4"): (167.4e6, "profiles/sep_tc_f16x5_c4.md"),
-    ("plain_f64_scalar", "c1"): (5.8e6, "profiles/plain_f64_scalar_c1.md"),
+    ("plain_f64_scalar", "c1"): (1.8e6, "profiles/plain_f64_fixed.md"),
     ("mixed_scalar", "c1"): (1.906e6, "profiles/mixed_fx_c1.md"),
     ("mixed_scalar", "c3"): (411.7e6 + 115.0e6, "profiles/mixed_fx_c3.md"),
     ("batch_mixed", "c5"): (2275.9e6 + 668.5e6, "profiles/batch_fx_c5.md"),
@@ -1126,6 +1127,15 @@ def _roofline_entry(args, w, dom, dom_ms, per_launch_units, op_mix, torch):
                 "peak_source": how,
                 "algorithmic_tflops_single_product": achieved / products,
                 "note": f"{products} split products x 2 x points x 2N FLOPs per launch"}
+    if dom == "sep_f64_slices":
+        flops = 26 * 2.0 * per_launch_units * 2 * (w["dim"] if w["incompr"] else 1)
+        achieved = flops / (dom_ms * 1e-3) / 1e12
+        peak = measured_peaks().get("bf16_tflops") or 1900.0
+        return {"bound": "tensor", "kernel": dom, "achieved": achieved, "peak": peak,
+                "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
+                "peak_source": "MEASURED_PEAKS.json bf16_tflops (fallback 1.9 PFLOP/s)",
+                "algorithmic_tflops_single_product": achieved / 26,
+                "note": "26 products of bf16 digits x 2 x points x 2N FLOPs per launch"}
     if op_mix is None:
         op_mix = {(w["dim"], bool(w["incompr"])): 1.0}
     # the algorithmic work per point*mode: 2d+3 FLOPs and one sincos (scalar),
@@ -1163,7 +1173,8 @@ def _roofline_entry(args, w, dom, dom_ms, per_launch_units, op_mix, torch):
             "traffic": None, "peak_source": how,
             "pipe_ops_per_point_mode": ops, "algorithmic": algo,
             "note": f"{ops:.1f} FP64 pipe instructions per point*mode "
-                    f"(from the kernel source), each counted as one FMA = 2 FLOPs"}
+                    f"(from the kernel source), each counted as one FMA = 2 FLOPs; "
+                    f"integer instructions beside them take about as long"}
 
 
 _PEAKS = {}

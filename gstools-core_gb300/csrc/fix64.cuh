@@ -212,6 +212,7 @@ __device__ __forceinline__ void cis_fine(uint64_t theta, int64_t *cosine, int64_
 // with factors of exponents within 200 are too small to matter to a phase.
 struct Factor {
     uint32_t m1, m0, e;
+    // the number itself (not of a zero)
     __device__ __forceinline__ double value() const {
         return __hiloint2double(static_cast<int>(e | ((m1 << 1) >> 12)),
                                 static_cast<int>(__funnelshift_r(m0, m1, 11)));

@@ -12,7 +12,9 @@
 //  * phase k.x with the reference's bits: ((k0*x0 + k1*x1) + k2*x2), no FMA
 //    (src/field.rs:57, src/short_vec.rs:30-33).  The first product and the sums
 //    are FP64 instructions; the other products are formed and rounded by
-//    integer instructions (rn_product), which overlap them;
+//    integer instructions (rn_product), which overlap them (in 2-D every
+//    second point of a thread has its second product on the FP64 pipe too, so
+//    that both kinds take about as long: 606 -> 598 us);
 //  * z1 cos + z2 sin = A cos(phase - beta), A = |z1 + i z2| and beta its
 //    angle, set up per mode (plain_rec_kernel); the phase becomes a 64-bit
 //    fraction of a turn and its cosine a 64-bit integer (fix64.cuh: 1.2e-16
@@ -23,7 +25,7 @@
 //    instructions per point*mode for d = 3 and 16 for d = 2; this one has 3 and
 //    2.  Integer issue bounds the kernel now (a mode's 110 to 190 integer
 //    instructions against 77 clocks for each FP64 one): 100,000 2-D points x
-//    1000 modes 3391 -> 620 us, 250,007 3-D points x 1999 modes 18.86 -> 3.54 ms
+//    1000 modes 3391 -> 598 us, 250,007 3-D points x 1999 modes 18.86 -> 3.53 ms
 //    (4.89 with all products on the FP64 pipe), and the error against 64-bit
 //    sums fell from 1.7e-15 to 7e-16;
 //  * phases of 2^32 and more, and modes with a NaN or an infinity, take CUDA's
