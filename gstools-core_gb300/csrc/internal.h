@@ -281,6 +281,7 @@ int sep_tc_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st);
 // (separable_f64.cu) queued behind for inputs outside their range; the FP64 MMA
 // alone for a call predicated on run_if
 int sep_f64_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st);
+int sep_f64_mma_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st);   // the FP64 MMA kernels alone
 int sep_slices_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st);
 // The FP64 MMA's scratch bytes, and its launches on scratch `base`, which do
 // nothing while *run_if is 0 (run_if null: always run)

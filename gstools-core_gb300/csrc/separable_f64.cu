@@ -295,6 +295,10 @@ int sep_f64_launch(const SepArgs &a, unsigned char *base, const int *run_if, cud
 int sep_f64_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
     if (a.n[0] * a.n[1] * (a.dim == 3 ? a.n[2] : 1) == 0) return GSC_OK;
     if (!a.run_if && a.n_modes > 0) return sep_slices_run(ctx, a, st);
+    return sep_f64_mma_run(ctx, a, st);
+}
+
+int sep_f64_mma_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
     GSC_TRY(ensure_dev(ctx, ctx.scratch, sep_f64_scratch(a)));
     GSC_CUDA(cudaStreamWaitEvent(st, ctx.scratch_ready, 0));
     GSC_TRY(sep_f64_launch(a, static_cast<unsigned char *>(ctx.scratch.ptr), a.run_if, st));

@@ -837,7 +837,7 @@ int sep_slices_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
         sms = 152;
     }
     const size_t out_bytes = sizeof(double) * static_cast<size_t>(ncomp) * P;
-    const SlPlan pl = sl_plan(rows, ncomp * nn, N, static_cast<int64_t>(out_bytes), sms);
+    SlPlan pl = sl_plan(rows, ncomp * nn, N, static_cast<int64_t>(out_bytes), sms);
     const int np = pl.kb * kKbModes;
 
     // scratch: words, modes, s, B, G images, F images of a slab, split fields;
@@ -848,11 +848,20 @@ int sep_slices_run(DeviceCtx &ctx, const SepArgs &a, cudaStream_t st) {
     const size_t off_g = up(off_b + sizeof(longlong2) * static_cast<size_t>(nm) * np, 1024);
     const size_t g_bytes = static_cast<size_t>(pl.n_tiles) * pl.kb * kSlices * pl.nt * 64;
     const size_t off_f = up(off_g + g_bytes, 1024);
-    const size_t f_bytes = static_cast<size_t>(pl.slab) * pl.kb * kSlices * kSliceF;
-    const size_t off_part = up(off_f + f_bytes, 1024);
-    const int parts = pl.splits > 1 ? pl.splits * pl.segs : 0;
-    const size_t total = std::max(off_part + parts * out_bytes, 256 + sep_f64_scratch(a));
-    GSC_TRY(ensure_dev(ctx, ctx.scratch, total));
+    size_t off_part = 0;
+    int parts = 0;
+    for (;;) {
+        off_part = up(off_f + static_cast<size_t>(pl.slab) * pl.kb * kSlices * kSliceF, 1024);
+        parts = pl.splits > 1 ? pl.splits * pl.segs : 0;
+        const int rc = ensure_dev(ctx, ctx.scratch, std::max(off_part + parts * out_bytes, 256 + sep_f64_scratch(a)));
+        if (rc == GSC_OK) break;
+        if (rc != GSC_ERR_NOMEM) return rc;
+        // no room: the digits of fewer rows at a time, then no splits, at last
+        // the FP64 MMA kernels, which need neither
+        if (pl.slab > 1) pl.slab = std::max<int64_t>(1, pl.slab / 4);
+        else if (pl.splits > 1) pl.splits = 1;
+        else return sep_f64_mma_run(ctx, a, st);
+    }
     GSC_CUDA(cudaStreamWaitEvent(st, ctx.scratch_ready, 0));
     unsigned char *base = static_cast<unsigned char *>(ctx.scratch.ptr);
 

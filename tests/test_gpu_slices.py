@@ -149,3 +149,30 @@ def test_device_call_and_replay(gsc):
     gsc.device_status()
     ref = oracle.summator(cov, z1, z2, _points(axes), num_threads=NT)
     assert np.max(np.abs(first - ref)) <= _tolerance(cov, z1, z2, axes)
+
+
+def test_smaller_slabs_when_memory_is_short(gsc):
+    """A call whose digits do not fit (the first allocation fails, injected on
+    the host) makes those of fewer rows at a time: the same bits."""
+    torch = pytest.importorskip("torch")
+    from gstools_core import _native
+    cov, z1, z2, axes = _inputs(10, (9, 130, 70), 200)
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    args = (d(cov), d(z1), d(z2), tuple(d(a) for a in axes))
+    outs = [torch.full((9 * 130 * 70,), float("nan"), dtype=torch.float64, device="cuda") for _ in range(2)]
+    stream = torch.cuda.current_stream()
+    gsc.release_buffers()
+    assert _native.lib.gsc_selftest_fail_alloc(0) == 0
+    try:
+        gsc.summate_structured_device(*args, outs[0], stream=stream.cuda_stream)
+    finally:
+        _native.lib.gsc_selftest_fail_alloc(-1)
+    stream.synchronize()
+    gsc.release_buffers()
+    gsc.summate_structured_device(*args, outs[1], stream=stream.cuda_stream)
+    stream.synchronize()
+    gsc.device_status()
+    a, b = (o.cpu().numpy() for o in outs)
+    assert np.array_equal(a, b)
+    ref = oracle.summator(cov, z1, z2, _points(axes), num_threads=NT)
+    assert np.max(np.abs(a - ref)) <= _tolerance(cov, z1, z2, axes)
