@@ -25,7 +25,7 @@
 //    instructions per point*mode for d = 3 and 16 for d = 2; this one has 3 and
 //    2.  Integer issue bounds the kernel now (a mode's 110 to 190 integer
 //    instructions against 77 clocks for each FP64 one): 100,000 2-D points x
-//    1000 modes 3391 -> 598 us, 250,007 3-D points x 1999 modes 18.86 -> 3.53 ms
+//    1000 modes 3391 -> 577 us, 250,007 3-D points x 1999 modes 18.86 -> 3.49 ms
 //    (4.89 with all products on the FP64 pipe), and the error against 64-bit
 //    sums fell from 1.7e-15 to 7e-16;
 //  * phases of 2^32 and more, and modes with a NaN or an infinity, take CUDA's
@@ -373,8 +373,8 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
 // dst + s*split_stride + i*sd + p*sp.
 // ---------------------------------------------------------------------------
 template <int D, int R, bool INC, bool LIBM>
-__global__ void __launch_bounds__(kThreads)
-plain_kernel(const double *__restrict__ pos, int64_t P, const double *__restrict__ rec, int64_t nc,
+__device__ __forceinline__ void
+plain_kernel_body(const double *__restrict__ pos, int64_t P, const double *__restrict__ rec, int64_t nc,
              int64_t mps, int accumulate, double *__restrict__ dst, int64_t sd, int64_t sp,
              int64_t split_stride, const int *__restrict__ run_if) {
     __shared__ PlainSmem sm;
@@ -389,6 +389,24 @@ plain_kernel(const double *__restrict__ pos, int64_t P, const double *__restrict
     plain_block<D, R, INC, LIBM>(pos, P, static_cast<int64_t>(blockIdx.x) * (kThreads * R), rec, jb, je,
                                  accumulate, dst + static_cast<int64_t>(blockIdx.y) * split_stride, sd,
                                  sp, sm);
+}
+template <int D, int R, bool INC, bool LIBM>
+__global__ void __launch_bounds__(kThreads)
+plain_kernel(const double *__restrict__ pos, int64_t P, const double *__restrict__ rec, int64_t nc,
+             int64_t mps, int accumulate, double *__restrict__ dst, int64_t sd, int64_t sp,
+             int64_t split_stride, const int *__restrict__ run_if) {
+    plain_kernel_body<D, R, INC, LIBM>(pos, P, rec, nc, mps, accumulate, dst, sd, sp, split_stride, run_if);
+}
+// Scalar fields with two points per thread: registers for more blocks per SM, since
+// more warps feed the FP64 pipe, up to where they spill.  100,000 2-D points x
+// 1000 modes 598 us at 8 blocks, 577 at 10; 250,007 3-D points x 1999 modes 3.52
+// ms at 7, 3.49 at 8, 3.52 at 9.
+template <int D>
+__global__ void __launch_bounds__(kThreads, D == 3 ? 8 : 10)
+plain_pair_kernel(const double *__restrict__ pos, int64_t P, const double *__restrict__ rec, int64_t nc,
+             int64_t mps, int accumulate, double *__restrict__ dst, int64_t sd, int64_t sp,
+             int64_t split_stride, const int *__restrict__ run_if) {
+    plain_kernel_body<D, 2, false, false>(pos, P, rec, nc, mps, accumulate, dst, sd, sp, split_stride, run_if);
 }
 
 // ---------------------------------------------------------------------------
@@ -500,8 +518,13 @@ int dispatch_dim(int64_t dim, dim3 grid, cudaStream_t st, const PlainLaunch &l) 
     if constexpr (!INC) {
         if (dim == 1) return launch(plain_kernel<1, R, INC, LIBM>);
     }
-    if (dim == 2) return launch(plain_kernel<2, R, INC, LIBM>);
-    if (dim == 3) return launch(plain_kernel<3, R, INC, LIBM>);
+    if constexpr (R == 2 && !INC && !LIBM) {
+        if (dim == 2) return launch(plain_pair_kernel<2>);
+        if (dim == 3) return launch(plain_pair_kernel<3>);
+    } else {
+        if (dim == 2) return launch(plain_kernel<2, R, INC, LIBM>);
+        if (dim == 3) return launch(plain_kernel<3, R, INC, LIBM>);
+    }
     return set_error(GSC_ERR_DIM, "unsupported dimension for the plain kernel");
 }
 
