@@ -180,16 +180,22 @@ int smem_attr(const void *fn, size_t smem) {
     });
 }
 
-// Allocation-failure injection (gsc_selftest_fail_alloc): -1 = off, k >= 0 =
-// the k-th next allocation of a library buffer fails as out of memory.
-static std::atomic<int> g_fail_alloc{-1};
+// Allocation-failure injection (gsc_selftest_fail_alloc, gsc_selftest_fail_allocs):
+// allocations of library buffers are counted up from 0 while it is on, and those
+// in [first, first + count) fail as out of memory.
+static std::atomic<int64_t> g_alloc_seen{0}, g_fail_first{0}, g_fail_end{0};
+
+static void inject_failures(int64_t first, int64_t count) {
+    g_fail_end.store(0);
+    g_alloc_seen.store(0);
+    g_fail_first.store(first);
+    g_fail_end.store(count > 0 ? first + count : 0);
+}
 
 static bool alloc_injected() {
-    int v = g_fail_alloc.load();
-    while (v >= 0) {
-        if (g_fail_alloc.compare_exchange_weak(v, v - 1)) return v == 0;
-    }
-    return false;
+    if (g_fail_end.load() == 0) return false;
+    const int64_t i = g_alloc_seen.fetch_add(1);
+    return i >= g_fail_first.load() && i < g_fail_end.load();
 }
 
 int alloc_device(void **p, size_t bytes, const char *what) {
@@ -1706,7 +1712,13 @@ int gsc_release_buffers(int32_t device) {
 
 int gsc_selftest_fail_alloc(int32_t countdown) {
     if (countdown < -1) return set_error(GSC_ERR_INVALID, "countdown must be -1 or >= 0");
-    g_fail_alloc.store(countdown);
+    inject_failures(countdown, countdown >= 0 ? 1 : 0);
+    return GSC_OK;
+}
+
+int gsc_selftest_fail_allocs(int32_t countdown, int32_t count) {
+    if (countdown < 0 || count < 0) return set_error(GSC_ERR_INVALID, "countdown and count must be >= 0");
+    inject_failures(countdown, count);
     return GSC_OK;
 }
 

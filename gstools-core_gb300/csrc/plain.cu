@@ -53,6 +53,7 @@ namespace {
 constexpr int kThreads = 128;                       // threads per block
 constexpr int kGroup = kPlainGroupModes;            // modes per staged tile and integer sum
 constexpr int64_t kChunkModes = 1 << 20;            // modes per record build
+constexpr int64_t kLeastChunkModes = 1 << 16;       // the same where device memory is short
 static_assert(kThreads == kBatchThreads, "batch units assume the plain block size");
 static_assert(kGroup == 32, "a warp builds the records of a group");
 
@@ -551,6 +552,12 @@ int dispatch_plain(int R, bool incompr, bool libm, int64_t dim, dim3 grid, cudaS
 // so an SM wants more than two blocks.  Small calls want the splits that give
 // them (1,000 2-D points x 1000 modes: 262 us with 2 splits at R = 2, 31 us with
 // 32 at R = 1), large ones whole waves.
+//
+// What splits smooth is part of one wave, a share that falls with the number of
+// waves, while their partial sums grow with the points: 28.8 million 3-D
+// vectors would gain 0.04 % from 2.8 GB of them.  They stop at
+// kMostPartialBytes, above what any call of up to 2 million points wants.
+constexpr int64_t kMostPartialBytes = int64_t(256) << 20;
 struct PlainShape {
     int R;
     int64_t bx, S, mps;
@@ -566,6 +573,7 @@ PlainShape plain_shape(int64_t P, int64_t chunk, int64_t dim, int64_t nout, int 
         const int64_t bx = (P + kThreads * R - 1) / (kThreads * R);
         for (int64_t S = 1; S <= 64 && S <= groups; ++S) {
             const int64_t per = (groups + S - 1) / S;
+            if (S > 1 && S * nout * P > kMostPartialBytes / static_cast<int64_t>(sizeof(double))) break;
             if ((groups + per - 1) / per != S) continue;       // fewer splits of the same share
             const double on_sm = std::ceil(static_cast<double>(bx) * S / sms);
             double cost = per * kGroup * std::max(on_sm, 2.2) * R * pm;
@@ -716,17 +724,26 @@ int plain_run(DeviceCtx &ctx, const PlainArgs &a, cudaStream_t st) {
         return set_error(GSC_ERR_DIM, "Only two- and three-dimensional problems are supported.");
 
     // ---- launch geometry ---------------------------------------------------
-    const int64_t chunk = std::min<int64_t>(N, kChunkModes);
-    const PlainShape shp = a.run_if ? plain_shape_unlikely(P, chunk, sm_count(ctx.device))
-                                    : plain_shape(P, chunk, dim, nout, sm_count(ctx.device), libm);
-    const int64_t S = shp.S;
+    int64_t chunk = std::min<int64_t>(N, kChunkModes);
+    PlainShape shp = a.run_if ? plain_shape_unlikely(P, chunk, sm_count(ctx.device))
+                              : plain_shape(P, chunk, dim, nout, sm_count(ctx.device), libm);
     if (shp.bx > 0x7fffffff) return set_error(GSC_ERR_INVALID, "too many points for one launch");
 
     // ---- scratch: mode records of one chunk, split partials ------------------
-    const size_t rec_bytes = static_cast<size_t>(chunk) * kPlainRecBytesPerMode;
-    const size_t part_bytes = S > 1 ? static_cast<size_t>(S) * nout * P * sizeof(double) : 0;
-    const size_t off_part = (rec_bytes + 255) / 256 * 256;
-    GSC_TRY(ensure_dev(ctx, ctx.scratch, off_part + part_bytes + 256));
+    size_t off_part = 0;
+    for (;;) {
+        off_part = (static_cast<size_t>(chunk) * kPlainRecBytesPerMode + 255) / 256 * 256;
+        const size_t part_bytes = shp.S > 1 ? static_cast<size_t>(shp.S) * nout * P * sizeof(double) : 0;
+        const int rc = ensure_dev(ctx, ctx.scratch, off_part + part_bytes + 256);
+        if (rc == GSC_OK) break;
+        if (rc != GSC_ERR_NOMEM) return rc;
+        // no room: no splits, then the records of fewer modes at a time
+        if (shp.S > 1) shp.S = 1;
+        else if (chunk > kLeastChunkModes) chunk = std::max<int64_t>(kLeastChunkModes, chunk / 4 / kGroup * kGroup);
+        else return rc;
+        if (shp.S == 1) shp.mps = (chunk + kGroup - 1) / kGroup * kGroup;
+    }
+    const int64_t S = shp.S;
     GSC_CUDA(cudaStreamWaitEvent(st, ctx.scratch_ready, 0));
     unsigned char *sbase = static_cast<unsigned char *>(ctx.scratch.ptr);
     double *rec = reinterpret_cast<double *>(sbase);
@@ -745,7 +762,7 @@ int plain_run(DeviceCtx &ctx, const PlainArgs &a, cudaStream_t st) {
 
     int64_t j0 = 0;
     do {
-        const int64_t nc = std::min<int64_t>(N - j0, kChunkModes);
+        const int64_t nc = std::min<int64_t>(N - j0, chunk);
         if (nc > 0) {
             TimedLaunch tl(st);
             tl.begin(K_MODE_TABLE);

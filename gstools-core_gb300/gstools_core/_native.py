@@ -174,6 +174,7 @@ SIGNATURES = {
     "gsc_selftest_wait_timeout": (ctypes.c_int, [_I32, _I64]),
     "gsc_selftest_pipe_rates": (ctypes.c_int, [_I32, ctypes.POINTER(ctypes.c_double)]),
     "gsc_selftest_fail_alloc": (ctypes.c_int, [_I32]),
+    "gsc_selftest_fail_allocs": (ctypes.c_int, [_I32, _I32]),
     "gsc_selftest_detect_grid": (ctypes.c_int, [_P, _I64, _I64, _I64, _I64,
                                                 ctypes.POINTER(ctypes.c_int64)]),
     "gsc_selftest_once_per_device": (ctypes.c_int, [_I32, _I32, _I32, ctypes.POINTER(_I64)]),

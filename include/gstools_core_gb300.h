@@ -459,6 +459,11 @@ int gsc_selftest_pipe_rates(int32_t device, double *rates);
  * counterpart. */
 int gsc_selftest_fail_alloc(int32_t countdown);
 
+/* The same for `count` allocations in a row, from the `countdown`-th next one
+ * on (count 0 switches the injection off): for calls that try again with less
+ * memory.  No reference counterpart. */
+int gsc_selftest_fail_allocs(int32_t countdown, int32_t count);
+
 /* Structured-mesh recognition of the point entry points, on host arrays
  * alone (no device is touched): for pos (dim, n_points) with element
  * strides, sets n_axes[0..2] to the axis lengths when the points are
