@@ -1560,7 +1560,9 @@ template <int K>
 __global__ void __launch_bounds__(kJoinThreads) sep_x5_join_kernel(const X5Params xp, int bnx) {
     __shared__ double tile_out[BM][kJoinColumns + 1];
     after_previous();
-    if (*xp.bound_flag) return;          // the call is recomputed
+    // The call is recomputed.  Other blocks may set the flag below meanwhile, so
+    // one answer is taken for the whole block, before its barrier.
+    if (__syncthreads_or(*xp.bound_flag)) return;
     const TcParams &p = xp.base;
     const int tile = xp.tile0 + xp.full_tiles + static_cast<int>(blockIdx.y);
     const int64_t r0 = static_cast<int64_t>(tile / p.n_tiles) * BM;
