@@ -104,7 +104,10 @@ __device__ __forceinline__ void rec_group(const double *__restrict__ cov, int64_
     uint64_t beta = 0;
     double amp = 0.0;                                            // A 2^-ez
     int ez = 0;
-    if (regular) mode_angle(z1, z2, &amp, &ez, &beta);
+    // at k = 0 the sine is 0 everywhere: its weight must not count in A, whose
+    // size sets the error
+    const bool still = k[0] == 0.0 && k[1] == 0.0 && k[2] == 0.0;
+    if (regular) mode_angle(z1, still ? 0.0 : z2, &amp, &ez, &beta);
     const int nout = incompr ? dim : 1;
     double a[3] = {incompr ? amp * w[0] : amp, amp * w[1], amp * w[2]};
     double scale[3] = {0.0, 0.0, 0.0};
