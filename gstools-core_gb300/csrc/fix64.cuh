@@ -10,6 +10,7 @@
 //   turn_fraction(ph)  |ph| < 2^32 as a fraction of a turn in units of 2^-64,
 //                      whole turns dropped (the mantissa times 96 bits of
 //                      2 / pi, shifted by the exponent), within 2^-60 turn;
+//   turn_fraction_far(ph)  the same for |ph| < 2^44, from 128 bits of 2 / pi;
 //   cos_fixed(theta)   the cosine of a turn fraction in units of 2^-62: one
 //                      of 256 table entries and polynomials in the remainder.
 //                      Over all phases the error is 1.2e-16 RMS, 4.2e-16 at
@@ -130,6 +131,20 @@ __device__ __forceinline__ uint64_t turn_fraction(double ph) {
     const uint32_t sign = static_cast<uint32_t>(static_cast<int32_t>(hi) >> 31);
     const uint32_t fh = __funnelshift_l(b, a, t) ^ sign, fl = __funnelshift_l(c, b, t) ^ sign;
     return (static_cast<uint64_t>(fh) << 32) | fl;
+}
+
+// As turn_fraction for |ph| < 2^44, within 2^-63 turn: the upper 128 bits of the
+// mantissa times 2^128 2 / pi, shifted.
+__device__ __forceinline__ uint64_t turn_fraction_far(double ph) {
+    constexpr uint64_t ch = 0xA2F9836E4E441529ull, cl = 0xFC2757D1F534DDC0ull;
+    const uint64_t bits = static_cast<uint64_t>(__double_as_longlong(ph));
+    const uint64_t m = (bits << 11) | (uint64_t(1) << 63);                 // 1.f, left-aligned
+    const uint64_t lo = m * ch, low = lo + __umul64hi(m, cl);              // bits 64..127 of the product
+    const uint64_t high = __umul64hi(m, ch) + (low < lo ? 1u : 0u);        // 128..191
+    // |ph| = m 2^(e - 63): the fraction starts at bit 129 - e of the product
+    const int s = 1088 - static_cast<int>((bits >> 52) & 0x7ffu);          // 65 - e, at least 22
+    const uint64_t f = s < 64 ? (high << (64 - s)) | (low >> s) : s < 128 ? high >> (s - 64) : 0u;
+    return f ^ static_cast<uint64_t>(static_cast<int64_t>(bits) >> 63);
 }
 
 // cos(2 pi (theta - kCosOffset) / 2^64) in units of 2^-62

@@ -28,8 +28,10 @@
 //    1000 modes 3391 -> 577 us, 250,007 3-D points x 1999 modes 18.86 -> 3.49 ms
 //    (4.89 with all products on the FP64 pipe), and the error against 64-bit
 //    sums fell from 1.7e-15 to 7e-16;
-//  * phases of 2^32 and more, and modes with a NaN or an infinity, take CUDA's
-//    sincos() and FP64 sums for that mode (the same test for a whole warp);
+//  * phases of 2^32 to 1e13 differ in how they are brought to a fraction of a
+//    turn (100,000 2-D points x 500 modes 362 us, with sincos() 3000); larger
+//    ones, and modes with a NaN or an infinity, take CUDA's sincos() and FP64
+//    sums for that mode (the same tests for a whole warp);
 //  * mode records (96 bytes) are staged 32 at a time into shared memory with
 //    cp.async double buffering; each thread keeps R points in registers;
 //  * when there are too few points to fill 152 SMs, the modes are split
@@ -70,7 +72,8 @@ constexpr int kRec = 20, kRecStaged = 12;
 enum { R_K0 = 0, R_M1 = 1, R_M2 = 2, R_EXP = 3, R_BETA = 4, R_A0 = 5, R_S0 = 8, R_KABS = 11,
        R_Z1 = 12, R_Z2 = 13, R_W0 = 14, R_K1 = 17, R_K2 = 18 };
 static_assert(kRec * 8 == kPlainRecBytesPerMode, "record layout");
-constexpr float kFastPhase = 4.29e9f;               // |k| |x| bound of the integer path, below 2^32
+constexpr float kFastPhase = 4.29e9f;               // |k| |x| bound of turn_fraction, below 2^32
+constexpr float kFarPhase = 1e13f;                  // that of turn_fraction_far, below 2^44
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
@@ -284,6 +287,17 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
         for (int r = 0; r < R; ++r)
 #pragma unroll
             for (int i = 0; i < NOUT; ++i) sum[r][i] = 2 * tm;
+        // a mode's amplitudes (R_A0 ...) times its cosine c at point r
+        auto add_term = [&](int r, int64_t c, const double (&av)[3]) {
+            const int32_t ch = static_cast<int32_t>(c >> 32);
+            const int32_t c0 = static_cast<int32_t>(static_cast<uint32_t>(c) >> 1);
+#pragma unroll
+            for (int i = 0; i < NOUT; ++i) {
+                const int32_t ah = __double2loint(av[i]), a0 = __double2hiint(av[i]);
+                sum[r][i] += static_cast<int64_t>(ah) * ch;
+                sum[r][i] += static_cast<int64_t>(__mulhi(ah, c0) + __mulhi(a0, ch)) << 1;
+            }
+        };
 #pragma unroll 1
         for (int m = 0; m < tm; ++m) {
             const double2 *mr = reinterpret_cast<const double2 *>(rc + m * kRecStaged);
@@ -313,15 +327,20 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
                         const bool fp64 = D == 2 && (r & 1);
                         ph = __dadd_rn(ph, fp64 ? __dmul_rn(k1, x1[r]) : rn_product(kf[d - 1], xf[r][d - 1]));
                     }
-                    const int64_t c = cos_fixed(turn_fraction(ph) + beta, &sm.tab);
-                    const int32_t ch = static_cast<int32_t>(c >> 32);
-                    const int32_t c0 = static_cast<int32_t>(static_cast<uint32_t>(c) >> 1);
+                    add_term(r, cos_fixed(turn_fraction(ph) + beta, &sm.tab), av);
+                }
+            } else if (!LIBM && kb * xbound < kFarPhase) {
+                const double *ex = rec + (t0 + m) * kRec;
+                const double k[3] = {ex[R_K0], ex[R_K1], ex[R_K2]};
+                const double av[3] = {ex[R_A0], ex[R_A0 + 1], ex[R_A0 + 2]};
+                const uint64_t beta = static_cast<uint64_t>(__double_as_longlong(ex[R_BETA]));
 #pragma unroll
-                    for (int i = 0; i < NOUT; ++i) {
-                        const int32_t ah = __double2loint(av[i]), a0 = __double2hiint(av[i]);
-                        sum[r][i] += static_cast<int64_t>(ah) * ch;
-                        sum[r][i] += static_cast<int64_t>(__mulhi(ah, c0) + __mulhi(a0, ch)) << 1;
-                    }
+                for (int r = 0; r < R; ++r) {
+                    const int64_t p = p0 + r * kThreads;
+                    double x[D];
+#pragma unroll
+                    for (int d = 0; d < D; ++d) x[d] = p < P ? pos[d * P + p] : 0.0;
+                    add_term(r, cos_fixed(turn_fraction_far(phase_of<D>(k, x)) + beta, &sm.tab), av);
                 }
             } else {
                 const double *ex = rec + (t0 + m) * kRec;
