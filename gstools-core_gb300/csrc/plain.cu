@@ -29,7 +29,7 @@
 //    (4.89 with all products on the FP64 pipe), and the error against 64-bit
 //    sums fell from 1.7e-15 to 7e-16;
 //  * phases of 2^32 to 1e13 differ in how they are brought to a fraction of a
-//    turn (100,000 2-D points x 500 modes 362 us, with sincos() 3000); larger
+//    turn (100,000 2-D points x 500 modes 388 us, with sincos() 3000); larger
 //    ones, and modes with a NaN or an infinity, take CUDA's sincos() and FP64
 //    sums for that mode (the same tests for a whole warp);
 //  * mode records (96 bytes) are staged 32 at a time into shared memory with
@@ -200,6 +200,12 @@ __device__ __forceinline__ double phase_of(const double *k, const double *x) {
     return ph;
 }
 
+// The cosine of a phase of 2^32 and more, a call: inlined it cost the sums of
+// ordinary phases 0.7 % (100,000 2-D points x 1000 modes 578.5 -> 582.7 us).
+__device__ __noinline__ int64_t far_cos(double ph, uint64_t beta, const CosTable *tab) {
+    return cos_fixed(turn_fraction_far(ph) + beta, tab);
+}
+
 struct PlainSmem {
     CosTable tab;
     __align__(16) double rec[2][kGroup * kRecStaged];
@@ -340,7 +346,7 @@ __device__ __forceinline__ void plain_block(const double *__restrict__ pos, int6
                     double x[D];
 #pragma unroll
                     for (int d = 0; d < D; ++d) x[d] = p < P ? pos[d * P + p] : 0.0;
-                    add_term(r, cos_fixed(turn_fraction_far(phase_of<D>(k, x)) + beta, &sm.tab), av);
+                    add_term(r, far_cos(phase_of<D>(k, x), beta, &sm.tab), av);
                 }
             } else {
                 const double *ex = rec + (t0 + m) * kRec;
