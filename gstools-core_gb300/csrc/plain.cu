@@ -559,7 +559,10 @@ int dispatch_dim(int64_t dim, dim3 grid, cudaStream_t st, const PlainLaunch &l) 
 
 int dispatch_plain(int R, bool incompr, bool libm, int64_t dim, dim3 grid, cudaStream_t st,
                    const PlainLaunch &l) {
-    if (libm)     // one launch shape: this form is a check on the others, not a fast path
+    if (libm && R == 1)
+        return incompr ? dispatch_dim<1, true, true>(dim, grid, st, l)
+                       : dispatch_dim<1, false, true>(dim, grid, st, l);
+    if (libm)
         return incompr ? dispatch_dim<4, true, true>(dim, grid, st, l)
                        : dispatch_dim<4, false, true>(dim, grid, st, l);
     if (R == 1)
@@ -579,7 +582,8 @@ int dispatch_plain(int R, bool incompr, bool libm, int64_t dim, dim3 grid, cudaS
 // and 3 % more at R = 4; a warp alone takes 2.2 times that per mode and point,
 // so an SM wants more than two blocks.  Small calls want the splits that give
 // them (1,000 2-D points x 1000 modes: 262 us with 2 splits at R = 2, 31 us with
-// 32 at R = 1), large ones whole waves.
+// 32 at R = 1), large ones whole waves.  CUDA's sincos() form has R = 1 and 4: one
+// 3-D point x 64 modes takes 52 and 169 us, 50,000 x 1000 modes 3157 and 3099.
 //
 // What splits smooth is part of one wave, a share that falls with the number of
 // waves, while their partial sums grow with the points: 28.8 million 3-D
@@ -596,8 +600,8 @@ PlainShape plain_shape(int64_t P, int64_t chunk, int64_t dim, int64_t nout, int 
     const double base = libm ? 2000.0 : nout > 1 ? (dim == 3 ? 350.0 : 280.0) : dim == 1 ? 195.0 : dim == 2 ? 250.0 : 295.0;
     const int64_t groups = std::max<int64_t>(1, (chunk + kGroup - 1) / kGroup);
     for (int R : {4, 2, 1}) {
-        if (libm && R != 4) continue;
-        const double pm = base * (R == 1 ? 1.07 : R == 2 ? 1.0 : 1.03);
+        if (libm && R == 2) continue;
+        const double pm = base * (libm ? (R == 1 ? 1.02 : 1.0) : R == 1 ? 1.07 : R == 2 ? 1.0 : 1.03);
         const int64_t bx = (P + kThreads * R - 1) / (kThreads * R);
         for (int64_t S = 1; S <= 64 && S <= groups; ++S) {
             const int64_t per = (groups + S - 1) / S;
