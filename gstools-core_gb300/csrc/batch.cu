@@ -476,14 +476,18 @@ std::vector<Cfg> candidates(const gsc_batch &b) {
 // the fastest per point*mode.  One pass of a sample varies by 2 % between runs,
 // as much as the best candidates differ, and the choice decides how the modes
 // are split, hence the last bits of the sums: candidates within 3 % of the
-// fastest are timed twice more, so that the same ensemble gets the same plan.
+// fastest are timed again, which makes it rarer (not impossible) that the same
+// ensemble gets another plan.  FP64 plans differ by 2 to 4 % and get four more
+// passes; mixed ones differ by less, and one more keeps their tuning at 12 to 16
+// passes (24 items of 40,000 points x 1500 modes: 10.9 ms of timed passes, 17.3 with
+// two rounds of an untimed and two timed ones, 9.1 with none).
 int autotune(gsc_batch &b, cudaStream_t st) {
     cudaEvent_t e0, e1;
     GSC_CUDA(cudaEventCreate(&e0));
     GSC_CUDA(cudaEventCreate(&e1));
     int rc = GSC_OK;
-    // the best rate of `passes` passes of candidate c, after an untimed one
-    auto time_candidate = [&](const Cfg &c, int passes, double *rate) -> int {
+    // the best rate of `passes` passes of candidate c, after an untimed one if `first`
+    auto time_candidate = [&](const Cfg &c, bool first, int passes, double *rate) -> int {
         *rate = -1.0;
         const int occ = occupancy(b, c);
         if (occ <= 0) return GSC_OK;
@@ -509,7 +513,7 @@ int autotune(gsc_batch &b, cudaStream_t st) {
         if (sample.empty() || work <= 0.0) return GSC_OK;
         GSC_TRY(upload_units(b, sample));
         const int64_t ns = static_cast<int64_t>(sample.size());
-        GSC_TRY(enqueue_sum(b, c, blocks, ns, st));      // the first launch of the instantiation
+        if (first) GSC_TRY(enqueue_sum(b, c, blocks, ns, st));      // the first launch of the instantiation
         float ms = 1e30f;
         for (int t = 0; t < passes; ++t) {
             GSC_CUDA(cudaEventRecord(e0, st));
@@ -527,17 +531,15 @@ int autotune(gsc_batch &b, cudaStream_t st) {
     const std::vector<Cfg> list = candidates(b);
     std::vector<double> rate(list.size(), -1.0);
     rc = enqueue_tables(b, st);
-    for (size_t k = 0; k < list.size() && rc == GSC_OK; ++k) rc = time_candidate(list[k], 2, &rate[k]);
-    for (int round = 0; round < 2 && rc == GSC_OK; ++round) {
-        const double top = *std::max_element(rate.begin(), rate.end());
-        if (std::count_if(rate.begin(), rate.end(), [&](double r) { return r >= 0.97 * top; }) < 2) break;
+    for (size_t k = 0; k < list.size() && rc == GSC_OK; ++k) rc = time_candidate(list[k], true, 2, &rate[k]);
+    const double top = *std::max_element(rate.begin(), rate.end());
+    if (std::count_if(rate.begin(), rate.end(), [&](double r) { return r >= 0.97 * top; }) > 1)
         for (size_t k = 0; k < list.size() && rc == GSC_OK; ++k) {
             if (rate[k] < 0.97 * top) continue;
             double r = -1.0;
-            rc = time_candidate(list[k], 2, &r);
+            rc = time_candidate(list[k], false, is_plain(b) ? 4 : 1, &r);
             rate[k] = std::max(rate[k], r);
         }
-    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (rc != GSC_OK) return rc;
