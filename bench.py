@@ -23,8 +23,8 @@ benchmark data):
       benches/input text format (--input-dir; synthesized stand-ins when
       absent); one step = the five calls
   all  [default] c1 .. c5 in turn; the JSON line is c5's (the largest
-      workload, 1.7e11 point*modes per step) with every workload's full
-      record under "configs" and a short "summary"
+      workload, 1.7e11 point*modes per step) with a "summary" of every
+      workload, whose full records go to stderr
 
 One step = one full summation of the workload.  `value` is timed with CUDA
 events on the launch stream, inputs resident in HBM, L2 flushed (a 256 MiB
@@ -1306,16 +1306,25 @@ def run_workload(args, world, rank, local, wname, cpu_seconds, form_arg):
 
 
 def run_all(args, world, rank, local):
-    """Every workload in turn; the headline's JSON record carries them all."""
+    """Every workload in turn.  The line printed on stdout is the headline's
+    record with a summary of the others; the full records go to stderr, one
+    line each (together they are some 30 KB, more than a log's last lines
+    keep)."""
     lines = {}
     for n in ALL_WORKLOADS:
         lines[n] = run_workload(args, world, rank, local, n,
                                 args.cpu_seconds if n == HEADLINE else args.cpu_seconds_other,
                                 "auto")
+        if rank == 0:
+            print(f"record {n}: {json.dumps(lines[n])}", file=sys.stderr, flush=True)
+    return headline_record(lines)
+
+
+def headline_record(lines):
+    """The headline's record of all workloads' records."""
     head = dict(lines[HEADLINE])
-    head["configs"] = lines
     head["config"] = dict(head["config"],
-                          workload=f"{HEADLINE} (headline; every workload under configs)")
+                          workload=f"{HEADLINE} (headline; the other workloads under summary)")
     fr = [l["error_vs_fp64_full"]["max_abs_over_rms"] for l in lines.values()
           if l.get("error_vs_fp64_full")]
     head["summary"] = {
