@@ -638,7 +638,10 @@ static void gather2(const double *src, int64_t s0, int64_t s1, int64_t rows, int
 constexpr int64_t kGridMinPoints = 4096;   // smaller grids are not worth routing
 // Up to this many points the calling thread checks the mesh itself, while the GPU
 // computes, instead of starting a thread for it.  With the inputs' one packed copy
-// (six before) a 100 x 100 mesh x 1000 modes went from 175 to 104 us a call.
+// (six before) a 100 x 100 mesh x 1000 modes went from 175 to 104 us a call.  The
+// line lies where the check is still shorter than what the GPU takes: 255 x 256
+// points 113 us a call, 260 x 260 with the thread 143; 40^3 120, 41 x 40 x 40 142;
+// at 1e-6 125 and 156.
 constexpr int64_t kGridInlinePoints = 1 << 16;
 
 // Runs f(begin, end) over [0, n) on up to max_threads host threads (one for
@@ -876,7 +879,7 @@ static int host_plain(const double *cov, int64_t cs_d, int64_t cs_n, const doubl
     const int64_t nout = incompr ? dim : 1;
 
     // AUTO on a flattened structured mesh: the separable forms on its axes
-    // (FP64 DMMA at the default tolerance, within the same 1e-12 bar)
+    // (the sliced FP64 form at the default tolerance, within the same 1e-12 bar)
     // The candidate axes come from the first coordinates' run lengths; the
     // check of every point (one read of the whole array on the host cores)
     // runs on a host thread while the GPU computes on the candidate axes.  A

@@ -180,8 +180,8 @@ __device__ __forceinline__ int64_t cos_fixed(uint64_t theta, const CosTable *tab
 }
 
 // cos and sin of 2 pi (theta - kFineOffset) / 2^64 in units of 2^-62, within
-// 1e-17: the same table with one more order of the cosine and 64-bit products,
-// for factor tables, where an error is shared by many sums.
+// 1e-17: the same table steps with one more order of the cosine and 64-bit
+// products, for factor tables, where an error is shared by many sums.
 //   1 - cos(step rho) = f1 rho^2 (1 - f2 rho^2 + f3 rho^4)
 //   sin(step rho)     = step rho (1 - f4 rho^2 + f5 rho^4)
 // with the Taylor coefficients f1 = step^2 / 2, f2 = step^2 / 12, f3 =
@@ -209,15 +209,8 @@ __device__ __forceinline__ void cis_from(uint64_t theta, int64_t c, int64_t s, i
     *cosine = c - (((__mul64hi(c, ver) >> 8) + __mul64hi(s, sn) + 8) >> 4);
     *sine = s - (((__mul64hi(s, ver) >> 8) - __mul64hi(c, sn) + 8) >> 4);
 }
-__device__ __forceinline__ void cis_fine(uint64_t theta, const CosTable *tab, int64_t *cosine, int64_t *sine) {
-    const uint32_t a = static_cast<uint32_t>(theta >> 56);
-    const uint4 e = tab->wide[a], g = tab->wide[(a + 192) & 255];
-    const int64_t c = static_cast<int64_t>((static_cast<uint64_t>(e.y) << 32) | e.x);
-    const int64_t s = static_cast<int64_t>((static_cast<uint64_t>(g.y) << 32) | g.x);
-    cis_from(theta, c, s, cosine, sine);
-}
-// The same without a table in shared memory: for one value per thread, two
-// reads of the quarter wave cost less than the table's set-up.
+// No table in shared memory: for one value per thread, two reads of the quarter
+// wave cost less than the table's set-up.
 __device__ __forceinline__ void cis_fine(uint64_t theta, int64_t *cosine, int64_t *sine) {
     const int a = static_cast<int>(theta >> 56);
     cis_from(theta, quarter_cos(a), quarter_cos(a - 64), cosine, sine);

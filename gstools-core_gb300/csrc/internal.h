@@ -38,8 +38,8 @@ inline int cuda_ok(cudaError_t e) { return e == cudaSuccess ? GSC_OK : cuda_fail
 // ---- kernel ids (gsc_kernel_name / gsc_last_timings) ----------------------
 enum KernelId : int32_t {
     K_MODE_TABLE = 0,      // per-mode angle tables and projector weights
-    K_PLAIN_SCALAR = 1,    // FP64 scalar summator, table-driven sincos
-    K_PLAIN_INCOMPR = 2,   // FP64 incompressible summator, table-driven sincos
+    K_PLAIN_SCALAR = 1,    // FP64 scalar summator, fixed-point cosine
+    K_PLAIN_INCOMPR = 2,   // FP64 incompressible summator, fixed-point cosine
     K_PLAIN_LIBM = 3,      // FP64 summators on CUDA's sincos()
     K_SPLIT_REDUCE = 4,    // ordered sum of mode-split partials
     K_GENERIC = 5,         // any dimension, one thread per point
@@ -222,7 +222,7 @@ struct PlainArgs {
     bool incompr;        // vector field (dim outputs) instead of scalar
     double *out;         // device
     int64_t out_sd, out_sp;  // element strides of out[i, p] (scalar: 0, 1)
-    int variant;         // 0 table-driven sincos, 1 CUDA sincos()
+    int variant;         // 0 fixed-point cosine, 1 CUDA sincos()
     // plain_run only: null, or a device word; every launch does nothing
     // while the word is 0 (a fallback queued behind another form's launches)
     const int *run_if = nullptr;

@@ -738,8 +738,9 @@ batch_fx_table_kernel(const BatchItem *__restrict__ items,
 // Persistent batch kernel (see batch_plain_kernel in plain.cu).  SCALAR:
 // an ensemble without incompressible items, whose kernel carries only the
 // scalar variants (fewer registers, so R = 8 keeps 3 blocks per SM).
-// The blocks per SM decide how a plan splits modes, and with that the last FP32
-// digits: they do not follow the compiler's register counts.
+// The blocks per SM, queried when a plan is made, decide how it splits modes, and
+// with that the last FP32 digits; the launch bounds hold them where the register
+// counts of one compiler or another would give fewer.
 template <int R, bool SCALAR>
 __global__ void __launch_bounds__(kFxThreads, R >= 8 ? (SCALAR ? 3 : 2) : R == 2 && SCALAR ? 5 : 4)
 batch_fx_kernel(const BatchItem *__restrict__ items, const BatchUnit *__restrict__ units,
@@ -895,8 +896,8 @@ int mixed_fx_run(DeviceCtx &ctx, const PlainArgs &a, int *range_flag, cudaStream
         // every candidate on this call's data, timed by events; the winner
         // then computes the result.  Eight points per thread fold their sums
         // half as often, so their results differ in the last FP32 digits: they
-        // must win by half a per cent, so that a near tie (3-D, thousands of
-        // modes: all within 0.1 %) gives the same digits in every process.
+        // must win by half a per cent, so that near ties (3-D, thousands of
+        // modes: all within 0.1 %) rarely give other digits in another process.
         GSC_TRY(build(0, chunk));
         cudaEvent_t e0, e1;
         GSC_CUDA(cudaEventCreate(&e0));

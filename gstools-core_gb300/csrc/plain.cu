@@ -579,9 +579,10 @@ int dispatch_plain(int R, bool incompr, bool libm, int64_t dim, dim3 grid, cudaS
 // multiple of the group of 32), by the time of the busiest SM.  Measured on
 // GB300: a point*mode keeps a quarter of an SM for 195, 250 and 295 clocks a warp
 // in 1, 2 and 3 dimensions (280 and 350 for vectors) at R = 2, 7 % more at R = 1
-// and 3 % more at R = 4; a warp alone takes 2.2 times that per mode and point,
-// so an SM wants more than two blocks.  Small calls want the splits that give
-// them (1,000 2-D points x 1000 modes: 262 us with 2 splits at R = 2, 31 us with
+// and 3 % more at R = 4 (scalar fields at R = 2 were given more blocks per SM since,
+// and take about 235 and 280 in 2 and 3 dimensions); a warp alone takes 2.2 times
+// that per mode and point, so an SM wants more than two blocks.  Small calls want
+// the splits that give them (1,000 2-D points x 1000 modes: 262 us with 2 splits at R = 2, 31 us with
 // 32 at R = 1), large ones whole waves.  CUDA's sincos() form has R = 1 and 4: one
 // 3-D point x 64 modes takes 52 and 169 us, 50,000 x 1000 modes 3157 and 3099.
 //

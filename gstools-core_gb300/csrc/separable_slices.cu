@@ -104,7 +104,7 @@ struct SlTab {
     longlong2 *btab;               // [nm][16 kb]       B, units 2^-62
     unsigned char *g;              // [tile][k-block][slice] images of nt rows x 64 bytes
     unsigned char *f;              // [row tile of the slab][k-block][slice] images of 128 rows x 64 bytes
-    int64_t row0, rows, rows_total;   // the slab
+    int64_t row0, rows_total;         // the slab's first row; rows of the output
     int *words;
 };
 
@@ -801,8 +801,11 @@ static SlPlan sl_plan(int64_t rows, int ncn, int64_t n_modes, int64_t out_bytes,
     s.segs = static_cast<int>((n_modes + kSegModes - 1) / kSegModes);
     const int64_t seg_modes = std::min<int64_t>(n_modes, kSegModes);
     s.kb = static_cast<int>((seg_modes + kKbModes - 1) / kKbModes);
-    // slabs of whole waves of tiles, about 1 GB of F digits each (an even share
-    // of the rows when all fit)
+    // slabs of whole waves of tiles, about 1 GB of F digits each or one wave (one
+    // column tile and 4096 modes: 1.9 GB), or all rows where those fit.  Shorter
+    // mode segments, which would keep a wave in 1 GB, cost 5 to 7 % (200 x 120 x 60
+    // x 4096 modes 1352 -> 1416 us).  The library keeps the scratch, as any other,
+    // until gsc_release_buffers
     const int64_t tile_bytes = static_cast<int64_t>(s.kb) * kSlices * kSliceF;
     s.slab = s.m_tiles;
     if (s.m_tiles * tile_bytes > (int64_t(1) << 30)) {

@@ -976,7 +976,8 @@ struct X5Layout {
     static constexpr int HC = BNX / 2;                   // columns per worker half
     // setmaxnreg split: workers hold HC FP32 totals; the narrower tile leaves
     // the control warps room (192^3 x 2048 modes, incompressible: 711 us with
-    // 184 / 136, 724 with 200 / 104, 735 with 200 / 80, which spill)
+    // 184 / 136, where the split-tile variant spills 16 bytes, 724 with
+    // 200 / 104, 735 with 200 / 80)
     static constexpr int WORK_REGS = BNX == 256 ? 216 : 184;
     static constexpr int CTRL_REGS = BNX == 256 ? 48 : 136;
     static_assert(4 * 32 * (2 * WORK_REGS + CTRL_REGS) <= X5_THREADS * X5_LAUNCH_REGS,

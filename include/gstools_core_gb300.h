@@ -148,7 +148,7 @@ const char *gsc_kernel_name(int32_t kernel_id);
 int gsc_device_status(int32_t device);
 
 /* Frees the scratch memory the library keeps on `device` (-1 = current)
- * between calls: the input/output, table and staging buffers of host- and
+ * between calls (a large FP64 grid keeps up to 4 GB): the input/output, table and staging buffers of host- and
  * device-pointer calls, their pinned host staging, and the cached plan of
  * gsc_summate_batch_f64.  Waits for the library's queued work first; the
  * next call allocates again.  Plans made with gsc_batch_create are the
@@ -344,9 +344,10 @@ typedef struct gsc_batch_item {
 } gsc_batch_item;
 
 /* Configuration of a plan.  Inputs (0 = let the autotuner choose):
- * points_per_thread (2, 4, 8), tile_modes (FP64 form: 8 or 16, with 2 or 4
- * points per thread), units_per_block (target work units per resident
- * block: how finely item modes are split).  gsc_batch_get_config fills all
+ * points_per_thread (2, 4, 8), tile_modes (FP64 form: 8 or 16, 16 with 2 or
+ * 4 points per thread only; accepted for callers that name it, the kernels
+ * stage 32 modes whatever it is), units_per_block (target work units per
+ * resident block: how finely item modes are split).  gsc_batch_get_config fills all
  * fields with what the plan uses. */
 typedef struct gsc_batch_config {
     int32_t struct_size;            /* sizeof(gsc_batch_config)              */
