@@ -8,7 +8,7 @@
 // (src/field.rs:37-65, :97-182 on the expanded grid) to FP64 round-off, for
 // any inputs.  At 1.1 TFLOP/s it is the way out for what the sliced form
 // (separable_slices.cu) does not take (values that are not finite, phases of
-// 1e13 and more, calls without modes) and for grids that the x5 form flagged:
+// 2^32 and more, calls without modes) and for grids that the x5 form flagged:
 // both launches of a call are queued behind the fast form's and leave at once
 // unless the word at run_if is set.  They run a fixed number of blocks, so that
 // leaving costs the launches alone; a block takes the next tile when it is done

@@ -43,7 +43,7 @@
 // kernel of its own writes them in the layout the MMA reads (12 bytes per real
 // element), for slabs of rows that bound the memory.
 //
-// Inputs that are not finite, phases of 1e13 and more and amplitudes beyond
+// Inputs that are not finite, phases of 2^32 and more and amplitudes beyond
 // 2^+-900 set a word that stops the launches that follow; the FP64 MMA kernels
 // queued behind run only then.
 #include <cuda_runtime.h>
@@ -75,8 +75,7 @@ constexpr int kAccCols = 96;               // TMEM columns between accumulators
 constexpr int kTmem = 512;
 constexpr int kThreads = 320;              // 8 worker warps, a copy warp, an MMA warp
 constexpr int kCopyWarp = 8, kMmaWarp = 9;
-constexpr double kPhaseLimit = 4.29e9;     // turn_fraction's range, just below 2^32
-constexpr double kFarPhaseLimit = 1e13;    // turn_fraction_far's, below 2^44
+constexpr float kPhaseLimit = 4.29e9f;     // turn_fraction's range, just below 2^32
 // k-blocks between drains of each accumulator (see above)
 __host__ __device__ constexpr int drain_period(int a) { return a == 0 ? 12 : a == 1 ? 4 : a == 2 ? 3 : 2; }
 
@@ -217,8 +216,8 @@ sl_tables_kernel(SlTab t, int64_t n_g, int64_t n_b, int64_t n_s) {
     bool bad = false;
     auto fraction = [&](int d, int j, double x) -> uint64_t {
         const double ph = __dmul_rn(t.cov[static_cast<int64_t>(d) * t.n_modes + j], x);
-        bad = bad || !(fabs(ph) < kFarPhaseLimit);
-        return fabs(ph) < kPhaseLimit ? turn_fraction(ph) : turn_fraction_far(ph);
+        bad = bad || !(fabs(ph) < static_cast<double>(kPhaseLimit));
+        return turn_fraction(ph);
     };
     int64_t i = static_cast<int64_t>(blockIdx.x) * kTabThreads + threadIdx.x;
     const int64_t b_g = (n_g + kTabThreads - 1) / kTabThreads * kTabThreads;

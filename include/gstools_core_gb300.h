@@ -89,7 +89,7 @@ extern "C" {
                                   RMS), as 9-bit slices summed exactly on
                                   tcgen05 tensor cores; the double-precision
                                   MMA for values that are not finite and
-                                  phases of 1e13 and more                    */
+                                  phases of 2^32 and more                    */
 
 /* ---- flags ----------------------------------------------------------- */
 #define GSC_FLAG_TIMING     1  /* record per-kernel CUDA-event timings      */
