@@ -34,8 +34,14 @@ namespace {
 constexpr int TM = 64, TN = 64, TK = 32;     // tile rows, columns, K per stage
 constexpr int LDS = TK + 1;                  // padded shared-memory row (doubles)
 constexpr int kF64Threads = 128;
-constexpr int kF64Grid = 152 * 4;            // blocks that fit at once
-constexpr int kF64TabGrid = 152 * 6;         // the same of the tables
+constexpr int kF64TabGrid = 152 * 6;         // blocks of the tables that fit at once
+// Blocks of the products on an SM: no more than it has tiles to compute, held to
+// that by shared memory that they do not use.  They are launched while the tables
+// still run, and where more of them fitted, they were placed several to an SM,
+// beside idle ones, and shared its FP64 pipe to the end (40 x 80 x 100 x 2000
+// modes, 160 tiles: 19.0 against 9.6 ms; 8 tiles took the time of 4).
+constexpr int kF64Sms = 152, kF64MostPerSm = 4;
+constexpr int kF64Smem[kF64MostPerSm] = {120 << 10, 80 << 10, 60 << 10, 0};   // of a block with 1, 2, 3, 4 on an SM
 
 struct F64Tab {
     const double *cov, *z1, *z2;
@@ -98,12 +104,9 @@ __device__ void f64_gtab_entry(const F64Tab &t, int64_t i) {
     t.g[static_cast<int64_t>(row) * t.k_pad + 2 * j + 1] = im;
 }
 
-// s, B and G tables: a fixed grid strides over all entries.  The products' blocks
-// may start only when the tables are done: those that came earlier, while tables
-// still filled the SMs, were placed several to an SM and shared its FP64 pipe to
-// the end (40 x 80 x 100 x 2000 modes, 160 tiles: 19.0 against 9.6 ms).
+// s, B and G tables: a fixed grid strides over all entries
 __global__ void __launch_bounds__(256) f64_tables_kernel(F64Tab t) {
-    wait_previous();
+    after_previous();
     if (t.run_if && *t.run_if == 0) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) *t.next = 0;
     const int64_t n1 = static_cast<int64_t>(t.nb) * t.n_modes, n2 = static_cast<int64_t>(t.n_modes) * t.nm;
@@ -114,7 +117,6 @@ __global__ void __launch_bounds__(256) f64_tables_kernel(F64Tab t) {
         else if (i < n1 + n2) f64_btab_entry(t, i - n1);
         else f64_gtab_entry(t, i - n1 - n2);
     }
-    next_may_start();
 }
 
 __device__ __forceinline__ void dmma_8x8x4(double &d0, double &d1, double a, double b) {
@@ -304,8 +306,12 @@ int sep_f64_launch(const SepArgs &a, unsigned char *base, const int *run_if, cud
     }
     TimedLaunch tl(st);
     tl.begin(K_SEP_F64);
-    GSC_CUDA(launch_after(sep_f64_kernel, dim3(static_cast<unsigned>(std::min<int64_t>(p.tiles, kF64Grid))),
-                          dim3(kF64Threads), 0, st, p));
+    const int per_sm = static_cast<int>(std::min<int64_t>(kF64MostPerSm, (p.tiles + kF64Sms - 1) / kF64Sms));
+    const int own = (TM + TN) * LDS * static_cast<int>(sizeof(double));
+    const size_t pad = static_cast<size_t>(std::max(0, kF64Smem[per_sm - 1] - own));
+    GSC_TRY(smem_attr(reinterpret_cast<const void *>(sep_f64_kernel), kF64Smem[0]));
+    GSC_CUDA(launch_after(sep_f64_kernel, dim3(static_cast<unsigned>(std::min<int64_t>(p.tiles, per_sm * kF64Sms))),
+                          dim3(kF64Threads), pad, st, p));
     tl.end();
     return GSC_OK;
 }

@@ -210,7 +210,6 @@ constexpr int kTabThreads = 256;
 __global__ void __launch_bounds__(kTabThreads)
 sl_tables_kernel(SlTab t, int64_t n_g, int64_t n_b, int64_t n_s) {
     after_previous();
-    if (t.words[0]) return;          // left to the FP64 MMA kernels already
     const int np = t.kb * kKbModes;
     const int ew = top_exponent(t.words[1]);
     bool bad = false;
