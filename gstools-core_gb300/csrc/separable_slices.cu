@@ -32,10 +32,11 @@
 // Small modes keep their precision: a mode's amplitude A_j and its column
 // factor share its distance from the largest amplitude (s is scaled up and G
 // down by 2^a_j, a_j half the exponents between them), and the columns of a
-// vector component are scaled by its largest projector weight.  A_j is what the
-// mode adds to the field: without z2 where k = 0 (its sine is 0), and for a vector
-// field with the exponent of its largest projector weight in it, so that a mode
-// along the first axis, which adds nothing, does not set the scale.
+// vector component are scaled by its largest projector weight.  A_j is about what
+// the mode adds to the field: without z2 where k = 0 (its sine is 0), and for a
+// vector field with the exponent of its projector weights in it where all are
+// weak, so that a mode along the first axis, which adds nothing, does not set the
+// scale.
 //
 // Tables: phases k x in FP64 (as separable_f64.cu forms them), their cosines
 // and sines in 64-bit fixed point (fix64.cuh), the products s B in 64-bit
@@ -113,6 +114,22 @@ __device__ __forceinline__ int ceil_exponent(double x) {
     return e - (fabs(x) == scale_pow2(0.5, e) ? 1 : 0);
 }
 
+// A mode whose projector weights are all weak (wmax the largest, 0: it adds nothing):
+// their exponent goes into A.  Weights from kWeakWeight on stay: A is then at most
+// 2^6 of what the mode adds.
+constexpr double kWeakWeight = 0x1p-6;
+__device__ __noinline__ void weak_mode(SlMode &m, double wmax) {
+    if (wmax == 0.0) {
+        m.amp = 0.0;
+        m.ea = -kWordBias;
+        return;
+    }
+    const int e = max(ceil_exponent(wmax), -200);
+    m.ez += e;
+    m.ea += e;
+    for (int c = 0; c < 3; ++c) m.w[c] = scale_pow2(m.w[c], -e);
+}
+
 // z1 + i z2 of every mode as amplitude and angle, projector weights and the
 // exponents of the largest.
 __global__ void __launch_bounds__(128) sl_modes_kernel(SlTab t) {
@@ -142,20 +159,15 @@ __global__ void __launch_bounds__(128) sl_modes_kernel(SlTab t) {
         m.amp = 0.0;
         m.beta = 0;
         const double wmax = t.incompr ? fmax(fabs(m.w[0]), fmax(fabs(m.w[1]), t.dim == 3 ? fabs(m.w[2]) : 0.0)) : 1.0;
-        if (!bad && wmax > 0.0) {
-            const bool still = k[0] == 0.0 && k[1] == 0.0 && k[2] == 0.0;
+        const bool still = k[0] == 0.0 && k[1] == 0.0 && k[2] == 0.0;
+        if (!bad) {
             mode_angle(z1, still ? 0.0 : z2, &m.amp, &m.ez, &m.beta);
             if (m.amp > 0.0) {
                 m.ea = m.ez + ceil_exponent(m.amp);            // A <= 2^ea
                 bad = m.ea < -900 || m.ea > 900;
-                const int e = max(ceil_exponent(wmax), -200);  // |w| <= 2^e, or far below any other mode
-                if (e != 0) {
-                    m.ez += e;
-                    m.ea += e;
-                    for (int c = 0; c < 3; ++c) m.w[c] = scale_pow2(m.w[c], -e);
-                }
-                top[0] = m.ea + kWordBias;
             }
+            if (wmax < kWeakWeight) weak_mode(m, wmax);
+            if (m.amp > 0.0) top[0] = m.ea + kWordBias;
             for (int c = 0; c < t.ncomp; ++c)
                 if (m.w[c] != 0.0) top[1 + c] = ceil_exponent(m.w[c]) + kWordBias;   // |w| <= 2^e
         }
