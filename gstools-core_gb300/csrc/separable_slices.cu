@@ -293,7 +293,10 @@ sl_tables_kernel(SlTab t, int64_t n_g, int64_t n_b, int64_t n_s) {
             t.svec[i] = v;
         }
     }
-    if (bad) t.words[0] = 1;
+    // set once or a few times: a store by every warp of a table whose phases are all too
+    // large takes longer than the table (5000 x 1 points x 200 modes: 750 us a call,
+    // 630 so)
+    if (bad && *static_cast<volatile int *>(t.words) == 0) t.words[0] = 1;
 }
 
 // a b + c d of values in units of 2^-62 (|.| <= 1), in units of 2^-60; the
