@@ -638,10 +638,9 @@ static void gather2(const double *src, int64_t s0, int64_t s1, int64_t rows, int
 constexpr int64_t kGridMinPoints = 4096;   // smaller grids are not worth routing
 // Up to this many points the calling thread checks the mesh itself, while the GPU
 // computes, instead of starting a thread for it.  With the inputs' one packed copy
-// (six before) a 100 x 100 mesh x 1000 modes went from 175 to 104 us a call.  The
-// line lies where the check is still shorter than what the GPU takes: 255 x 256
-// points 113 us a call, 260 x 260 with the thread 143; 40^3 120, 41 x 40 x 40 142;
-// at 1e-6 125 and 156.
+// (six before) a 100 x 100 mesh x 1000 modes went from 175 to 104 us a call.  Up to
+// the line the thread costs more than it saves: 255 x 256 points 113 us a call, 260 x
+// 260 with the thread 143; 40^3 120, 41 x 40 x 40 142; at 1e-6 125 and 156.
 constexpr int64_t kGridInlinePoints = 1 << 16;
 
 // Runs f(begin, end) over [0, n) on up to max_threads host threads (one for
