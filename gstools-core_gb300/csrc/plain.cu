@@ -582,9 +582,10 @@ int dispatch_plain(int R, bool incompr, bool libm, int64_t dim, dim3 grid, cudaS
 // and 3 % more at R = 4 (scalar fields at R = 2 were given more blocks per SM since,
 // and take about 235 and 280 in 2 and 3 dimensions); a warp alone takes 2.2 times
 // that per mode and point, so an SM wants more than two blocks.  Small calls want
-// the splits that give them (1,000 2-D points x 1000 modes: 262 us with 2 splits at R = 2, 31 us with
-// 32 at R = 1), large ones whole waves.  CUDA's sincos() form has R = 1 and 4: one
-// 3-D point x 64 modes takes 52 and 169 us, 50,000 x 1000 modes 3157 and 3099.
+// the splits that give them (1,000 2-D points x 1000 modes: 262 us with 2 splits at
+// R = 2, 31 us with 32 at R = 1), large ones whole waves.  CUDA's sincos() form has
+// R = 1 and 4: one 3-D point x 64 modes takes 52 and 169 us, 50,000 x 1000 modes
+// 3157 and 3099.
 //
 // What splits smooth is part of one wave, a share that falls with the number of
 // waves, while their partial sums grow with the points: 28.8 million 3-D
